@@ -172,13 +172,12 @@ cudaError_t upload_views(CaelixBatch* b, const CaelixBatchTuning& t, uint32_t* i
     if (run_kernel(b, t) != CAELIX_BATCH_WAVEFRONT) return cudaSuccess;
     // The wavefront organisation: its view table, wave plan and path state.
     CX_TRY(cudaMemcpy(b->d_wave_views, b->wave_views.data(), sizeof(cx::WaveView) * n, cudaMemcpyHostToDevice));
-    b->plan = cx::wave_plan(b->wave_views.data(), n, bw);
+    const uint32_t most = t.wavefront ? t.wavefront : kDefaultWaveSlots;
+    b->plan = cx::wave_plan(b->wave_views.data(), n, bw, most);
     if (b->wave_table.reserve(4ull * std::max<size_t>(b->plan.table.size(), 1), "caelix_batch_run") != CAELIX_OK)
         return cudaErrorMemoryAllocation;
     CX_TRY(cudaMemcpy(b->wave_table.ptr, b->plan.table.data(), 4 * b->plan.table.size(), cudaMemcpyHostToDevice));
-    uint32_t largest = 0;
-    for (uint32_t w : b->plan.items) largest = std::max(largest, w);
-    const uint32_t slots = std::min(largest, t.wavefront ? t.wavefront : kDefaultWaveSlots);
+    const uint32_t slots = std::min(b->plan.largest(), most);
     if (b->wave_memory.reserve(cx::wave_buffer_bytes(slots), "caelix_batch_run") != CAELIX_OK)
         return cudaErrorMemoryAllocation;
     return cudaSuccess;
@@ -186,9 +185,7 @@ cudaError_t upload_views(CaelixBatch* b, const CaelixBatchTuning& t, uint32_t* i
 
 uint32_t wave_slots(const CaelixBatch* b, const CaelixBatchTuning& t)
 {
-    uint32_t largest = 0;
-    for (uint32_t w : b->plan.items) largest = std::max(largest, w);
-    return std::max(32u, std::min(largest, t.wavefront ? t.wavefront : kDefaultWaveSlots));
+    return std::max(32u, std::min(b->plan.largest(), t.wavefront ? t.wavefront : kDefaultWaveSlots));
 }
 
 uint32_t trace_grid(const CaelixBatch* b, const CaelixBatchTuning& t)

@@ -1275,8 +1275,8 @@ CAELIX_API CaelixResult caelix_renderer_render(CaelixRenderer* renderer, const C
         cudaEventRecord(renderer->stop, stream);
         renderer->launches = 1;
     } else {
-        // The wavefront trace of the one view: its path state sized for one sample of every pixel
-        // (or the set capacity), the view and its wave table uploaded ahead of the kernels.
+        // The wavefront trace of the one view: its path state sized for the samples of every pixel
+        // that one wave takes (or the set capacity), the view and its wave table uploaded ahead of the kernels.
         cx::WaveView view;
         std::memset(&view, 0, sizeof(view));
         view.scene = render_view(scene);
@@ -1285,10 +1285,19 @@ CAELIX_API CaelixResult caelix_renderer_render(CaelixRenderer* renderer, const C
         view.ray_counts = renderer->counts;
         constexpr uint32_t kBlockWidth = 8;  // 8 x 4 pixel blocks per warp
         view.blocks_x = (p.width + kBlockWidth - 1) / kBlockWidth;
-        const cx::WavePlan plan = cx::wave_plan(&view, 1, kBlockWidth);
-        const uint32_t items = plan.items.empty() ? 0 : plan.items[0];
-        const uint32_t capacity = renderer->wave_capacity ? std::min(renderer->wave_capacity, items) : items;
-        CaelixResult r2 = renderer->wave_memory.reserve(cx::wave_buffer_bytes(capacity), "caelix_renderer_render");
+        cx::WavePlan plan = cx::wave_plan(&view, 1, kBlockWidth, cx::wave_merge_slots(renderer->wave_capacity));
+        const auto slots_of = [&](const cx::WavePlan& w) {
+            return renderer->wave_capacity ? std::min(renderer->wave_capacity, w.largest()) : w.largest();
+        };
+        CaelixResult r2 =
+            renderer->wave_memory.reserve(cx::wave_buffer_bytes(slots_of(plan)), "caelix_renderer_render");
+        if (r2 == CAELIX_ERROR_OUT_OF_MEMORY) {
+            // One sample index per wave where the path state of several does not fit.
+            cudaGetLastError();
+            plan = cx::wave_plan(&view, 1, kBlockWidth, 0);
+            r2 = renderer->wave_memory.reserve(cx::wave_buffer_bytes(slots_of(plan)), "caelix_renderer_render");
+        }
+        const uint32_t capacity = slots_of(plan);
         const uint64_t view_bytes = (sizeof(cx::WaveView) + 255) & ~uint64_t{255};
         if (r2 == CAELIX_OK)
             r2 = renderer->wave_views.reserve(view_bytes + 4ull * plan.table.size(), "caelix_renderer_render");
@@ -1336,14 +1345,21 @@ CAELIX_API CaelixResult caelix_renderer_backward(CaelixRenderer* renderer, const
     if (e == cudaSuccess) e = cudaMemsetAsync(d_power, 0, sizeof(float) * std::max(scene->dev.brick_count, 1u), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(renderer->counts, 0, 24, stream);
     if (e != cudaSuccess) return cx::cuda_result(e, "caelix_renderer_backward");
-    const CaelixResult r2 =
-        renderer->wave_memory.reserve(cx::adjoint_bytes(p, renderer->wave_capacity), "caelix_renderer_backward");
+    uint32_t merge = cx::wave_merge_slots(renderer->wave_capacity);
+    CaelixResult r2 =
+        renderer->wave_memory.reserve(cx::adjoint_bytes(p, renderer->wave_capacity, merge), "caelix_renderer_backward");
+    if (r2 == CAELIX_ERROR_OUT_OF_MEMORY) {
+        // One sample index per wave where the path state of several does not fit.
+        cudaGetLastError();
+        merge = 0;
+        r2 = renderer->wave_memory.reserve(cx::adjoint_bytes(p, renderer->wave_capacity, merge), "caelix_renderer_backward");
+    }
     if (r2 != CAELIX_OK) return r2;
     renderer->launches = 0;
     cudaEventRecord(renderer->start, stream);
     e = cx::adjoint_launch(render_view(scene), p, d_radiance, reinterpret_cast<float*>(image), d_albedo,
                            d_power, renderer->counts, renderer->wave_memory.ptr, renderer->wave_capacity,
-                           renderer->device->sm_count, stream, &renderer->launches);
+                           merge, renderer->device->sm_count, stream, &renderer->launches);
     cudaEventRecord(renderer->stop, stream);
     renderer->last_stream = stream;
     renderer->frame_number = frame->frame_number;

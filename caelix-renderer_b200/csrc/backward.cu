@@ -36,24 +36,30 @@ constexpr uint32_t kAdjointBlockWidth = 8;
 
 uint64_t align256(uint64_t x) { return (x + 255u) & ~uint64_t{255}; }
 
+uint32_t plan_capacity(const WavePlan& plan, uint32_t wave_capacity)
+{
+    const uint32_t items = std::max(plan.largest(), 32u);
+    return wave_capacity ? std::min(wave_capacity, items) : items;
+}
+
 }  // namespace
 
-uint64_t adjoint_bytes(const TraceParams& p, uint32_t wave_capacity)
+uint64_t adjoint_bytes(const TraceParams& p, uint32_t wave_capacity, uint32_t merge_slots)
 {
     WaveView v;
     std::memset(&v, 0, sizeof(v));
     v.params = p;
     v.blocks_x = (p.width + kAdjointBlockWidth - 1) / kAdjointBlockWidth;
-    const WavePlan plan = wave_plan(&v, 1, kAdjointBlockWidth);
-    const uint32_t items = plan.items.empty() ? 32 : plan.items[0];
-    const uint32_t capacity = wave_capacity ? std::min(wave_capacity, items) : items;
+    const WavePlan plan = wave_plan(&v, 1, kAdjointBlockWidth, merge_slots);
+    const uint32_t capacity = plan_capacity(plan, wave_capacity);
     return 2 * align256(sizeof(WaveView)) + align256(4ull * plan.table.size()) +
            align256(12ull * p.spp * p.width * p.height) + wave_buffer_bytes(capacity);
 }
 
 cudaError_t adjoint_launch(const SceneView& s, const TraceParams& p, const float* d_radiance, float* image,
                            float* d_albedo, float* d_power, unsigned long long* ray_counts, void* memory,
-                           uint32_t wave_capacity, uint32_t sm_count, cudaStream_t stream, uint32_t* launches)
+                           uint32_t wave_capacity, uint32_t merge_slots, uint32_t sm_count, cudaStream_t stream,
+                           uint32_t* launches)
 {
     WaveView views[2];
     std::memset(views, 0, sizeof(views));
@@ -65,9 +71,8 @@ cudaError_t adjoint_launch(const SceneView& s, const TraceParams& p, const float
     views[1] = views[0];
     views[1].radiance = nullptr;    // the replay writes no image
     views[1].ray_counts = nullptr;  // and counts no rays
-    const WavePlan plan = wave_plan(views, 1, kAdjointBlockWidth);
-    const uint32_t items = plan.items.empty() ? 32 : plan.items[0];
-    const uint32_t capacity = wave_capacity ? std::min(wave_capacity, items) : items;
+    const WavePlan plan = wave_plan(views, 1, kAdjointBlockWidth, merge_slots);
+    const uint32_t capacity = plan_capacity(plan, wave_capacity);
     char* m = static_cast<char*>(memory);
     WaveView* d_record = reinterpret_cast<WaveView*>(m);
     m += align256(sizeof(WaveView));

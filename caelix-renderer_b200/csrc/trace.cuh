@@ -38,16 +38,19 @@ cudaError_t trace_launch(const SceneView& s, const TraceParams& p, float* radian
 // d_albedo (kMaterialCodes x 3, per material code) and d_power (one per brick, the scene's order) are accumulated
 // into (zero them first); image (may be null) receives the forward radiance; ray_counts (may be
 // null) the rays of the recording pass. `memory`: adjoint_bytes(p, wave_capacity) bytes of device
-// memory, 256-aligned (wave_capacity 0 = one path per pixel).
-uint64_t adjoint_bytes(const TraceParams& p, uint32_t wave_capacity);
+// memory, 256-aligned (wave_capacity 0 = a path for every item of the largest wave; merge_slots:
+// the wave plan's `slots`, wave_merge_slots(wave_capacity) or 0 for one sample index per wave).
+uint64_t adjoint_bytes(const TraceParams& p, uint32_t wave_capacity, uint32_t merge_slots);
 cudaError_t adjoint_launch(const SceneView& s, const TraceParams& p, const float* d_radiance, float* image,
                            float* d_albedo, float* d_power, unsigned long long* ray_counts, void* memory,
-                           uint32_t wave_capacity, uint32_t sm_count, cudaStream_t stream, uint32_t* launches);
+                           uint32_t wave_capacity, uint32_t merge_slots, uint32_t sm_count, cudaStream_t stream,
+                           uint32_t* launches);
 
 // ---- the wavefront trace (wave.cu) ----
 //
-// Paths live in HBM (structure of arrays, one slot per path); a wave is every pixel of one sample
-// index of the views that have it, split into sub-waves of at most `capacity` slots. Per bounce
+// Paths live in HBM (structure of arrays, one slot per path); a wave is every pixel of one or more
+// consecutive sample indices of the views that have them (WavePlan), a wave of one sample index
+// split into sub-waves of at most `capacity` slots. Per bounce
 // two kernels run over compacted queues: wave_trace_kernel traces every queued ray (extension
 // and shadow rays alike, one DDA code path) and wave_shade_kernel advances every live path by
 // one vertex (shadow result, emission and MIS, albedo, light-tree NEE, Russian roulette),
@@ -106,17 +109,35 @@ struct WaveAdjoint
 uint64_t wave_buffer_bytes(uint32_t capacity);
 WaveBuffers wave_carve(void* base, uint32_t capacity);
 
-// The wave plan of a set of views: for every sample index s below the largest spp, the views
-// with spp > s and their first item (pixel blocks x 32 per view) in that wave.
+// The wave plan of a set of views. A wave holds the samples [first, first + samples) of the views
+// with spp > first (every one of them has all these samples): its entries are (view, sample) pairs,
+// sample by sample, each with its first item (pixel blocks x 32 per entry). More than one sample
+// index joins a wave while its items fit `slots` (they are then all in flight at once); a wave of
+// one sample index may be larger.
+//
+// A wave of few paths leaves the chip idle: a launch lasts as long as its longest ray, and one
+// sample of a 256 x 256 frame is 65,536 paths on 148 SMs. Measured (one B200), one wave per sample
+// index against several in one wave: 333 x 251, 8 spp 3.65 against 1.48 ms; the adjoint of 256 x 256,
+// 8 spp 7.60 against 3.83 ms; 1920 x 1080, 4 spp (8.3 M paths at once) 25.5 against 20.4 ms. Fewer
+// slots: 1.78 ms for the first at 512 k (two waves), 25.2-27.1 ms for the last at 1 M and 2 M (it
+// then runs one sample at a time). At 2^23 slots the path state is 2.1 GB, of 180.
 struct WavePlan
 {
-    std::vector<uint32_t> table;     // per wave: view indices, then item bases (n_views each)
-    std::vector<uint32_t> offset;    // per wave: first word of its views in `table`
-    std::vector<uint32_t> views;     // per wave: number of views
+    std::vector<uint32_t> table;     // per wave: entries (view | sample << 16), then item bases
+    std::vector<uint32_t> offset;    // per wave: first word of its entries in `table`
+    std::vector<uint32_t> entries;   // per wave: number of entries
+    std::vector<uint32_t> samples;   // per wave: sample indices
     std::vector<uint32_t> items;     // per wave: items
     std::vector<uint32_t> bounces;   // per wave: the largest bounce count of its views
+    uint32_t largest() const;        // the items of the largest wave
 };
-WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_width);
+constexpr uint32_t kWaveMergeSlots = 1u << 23;
+WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_width, uint32_t slots);
+// The plan's `slots` for a single view's render or adjoint with a wave capacity (0: not set).
+inline uint32_t wave_merge_slots(uint32_t wave_capacity)
+{
+    return wave_capacity && wave_capacity < kWaveMergeSlots ? wave_capacity : kWaveMergeSlots;
+}
 
 // Records the trace of every sample of every view into `stream` (no host synchronisation):
 // d_views the device copy of `views`, d_table the device copy of plan.table. The views'

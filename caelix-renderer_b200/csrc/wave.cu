@@ -47,9 +47,9 @@ __device__ __forceinline__ uint32_t fetch_chunk(uint32_t* counter)
 
 struct WaveGen
 {
-    const uint32_t* table;  // view indices, then item bases (n_views each)
-    uint32_t n_views;
-    uint32_t sample;
+    const uint32_t* table;  // entries (view | sample << 16), then item bases (`entries` each)
+    uint32_t entries;
+    uint32_t samples;  // sample indices of the wave
     uint32_t first_item;
     uint32_t count;
     uint32_t block_width;
@@ -72,6 +72,20 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, uint32_t n)
     return base + incl - n;
 }
 
+// The entry (of the first `entries` of a wave) that holds item `item`, and the item within it.
+__device__ __forceinline__ uint32_t wave_entry(const WaveGen& g, uint32_t entries, uint32_t item, uint32_t& local)
+{
+    const uint32_t* bases = g.table + g.entries;
+    uint32_t lo = 0, hi = entries;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(bases + mid) <= item) lo = mid;
+        else hi = mid;
+    }
+    local = item - __ldg(bases + lo);
+    return lo;
+}
+
 __global__ void __launch_bounds__(kWaveThreads)
     wave_generate_kernel(const WaveView* __restrict__ views, const WaveGen g, const WaveBuffers b)
 {
@@ -80,17 +94,10 @@ __global__ void __launch_bounds__(kWaveThreads)
     bool valid = false;
     if (i < g.count) {
         const uint32_t item = g.first_item + i;
-        const uint32_t* bases = g.table + g.n_views;
-        uint32_t lo = 0, hi = g.n_views;
-        while (hi - lo > 1u) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(bases + mid) <= item) lo = mid;
-            else hi = mid;
-        }
-        const uint32_t v = __ldg(g.table + lo);
-        const WaveView& V = views[v];
+        uint32_t local;
+        const uint32_t vs = __ldg(g.table + wave_entry(g, g.entries, item, local));
+        const WaveView& V = views[vs & 0xFFFFu];
         const TraceParams& P = V.params;
-        const uint32_t local = item - __ldg(bases + lo);
         const uint32_t blk = local >> 5, in = local & 31u;
         const uint32_t px = (blk % V.blocks_x) * bw + in % bw;
         const uint32_t py = (blk / V.blocks_x) * bh + in / bw;
@@ -109,7 +116,7 @@ __global__ void __launch_bounds__(kWaveThreads)
 #pragma unroll
             for (int k = 0; k < 3; ++k) d[k] = d[k] * inv_len;
             b.item[i] = py * P.width + px;
-            b.vs[i] = v | (g.sample << 16);
+            b.vs[i] = vs;
             b.flags[i] = kFlagExt | kFlagPrimary;
             b.org[i] = make_float4(P.position[0], P.position[1], P.position[2], 0.0f);
             b.dir[i] = make_float4(d[0], d[1], d[2], 0.0f);
@@ -121,6 +128,45 @@ __global__ void __launch_bounds__(kWaveThreads)
         b.pathq[0][q] = i;
         b.rayq[0][r] = i | (kKindPrimary << 30);
     }
+}
+
+// A wave of several sample indices: its finished paths left their samples' values in the slots
+// (b.radiance); one thread per pixel adds them to the radiance buffer in sample order (the sums of
+// the waves of one sample index, bit for bit), and divides with the last sample. Bound by its reads,
+// 16 bytes per sample and 12 written per pixel, coalesced.
+__global__ void __launch_bounds__(kWaveThreads)
+    wave_resolve_kernel(const WaveView* __restrict__ views, const WaveGen g, const WaveBuffers b)
+{
+    const uint32_t n_views = g.entries / g.samples;
+    const uint32_t item = blockIdx.x * kWaveThreads + threadIdx.x;
+    const uint32_t per_sample = g.count / g.samples;
+    if (item >= per_sample) return;
+    const uint32_t bw = g.block_width, bh = 32u / bw;
+    uint32_t local;
+    const uint32_t vs = __ldg(g.table + wave_entry(g, n_views, item, local));
+    const WaveView& V = views[vs & 0xFFFFu];
+    const TraceParams& P = V.params;
+    if (!V.radiance) return;
+    const uint32_t blk = local >> 5, in = local & 31u;
+    const uint32_t px = (blk % V.blocks_x) * bw + in % bw;
+    const uint32_t py = (blk / V.blocks_x) * bh + in / bw;
+    if (px >= P.width || py >= P.height) return;
+    const uint32_t first = vs >> 16;
+    float* o = V.radiance + 3ull * (py * P.width + px);
+    float acc[3] = {0.0f, 0.0f, 0.0f};
+    if (first != 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k] = o[k];
+    }
+    for (uint32_t s = 0; s < g.samples; ++s) {
+        const float4 r = b.radiance[item + s * per_sample];
+        acc[0] += r.x;
+        acc[1] += r.y;
+        acc[2] += r.z;
+    }
+    const bool last = first + g.samples == P.spp;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o[k] = last ? acc[k] / (float)P.spp : acc[k];
 }
 
 // kEntities: the views' scenes have entities (traversed after the world's bricks); the variant
@@ -214,10 +260,12 @@ struct AlbedoCache
 // in flight hide them (measured: 5 is the fastest of 3 .. 8 on the 128^3 world; 8 on the
 // 2 M-brick world and the 64-scene batch).
 // kEntities: the views' scenes have entities (their hits, their lights); the variant without
-// them keeps the world-only shading's registers.
+// them keeps the world-only shading's registers. resolve: a finished path leaves its sample in its
+// slot for wave_resolve_kernel (several samples of a pixel are in flight).
 template <int kMode, int kMinBlocks, bool kEntities>
 __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
-    wave_shade_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj)
+    wave_shade_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj,
+                      bool resolve)
 {
     __shared__ float s_albedo[kMode == kShadeReplay ? kAlbedoCache * 3 : 1];
     __shared__ uint32_t s_tag[kMode == kShadeReplay ? kAlbedoCache : 1];
@@ -485,12 +533,16 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
                         rgb[k] = e0[k] + a0[k] * sr;
                     }
                 }
-                float* o = V.radiance + 3ull * item;
-                const bool last = sp + 1u == P.spp;
+                if (resolve) {
+                    b.radiance[slot] = make_float4(rgb[0], rgb[1], rgb[2], 0.0f);
+                } else {
+                    float* o = V.radiance + 3ull * item;
+                    const bool last = sp + 1u == P.spp;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float acc = (sp == 0 ? 0.0f : o[k]) + rgb[k];
-                    o[k] = last ? acc / (float)P.spp : acc;
+                    for (int k = 0; k < 3; ++k) {
+                        const float acc = (sp == 0 ? 0.0f : o[k]) + rgb[k];
+                        o[k] = last ? acc / (float)P.spp : acc;
+                    }
                 }
             }
         }
@@ -561,31 +613,49 @@ WaveBuffers wave_carve(void* base, uint32_t capacity)
     return b;
 }
 
-WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_width)
+uint32_t WavePlan::largest() const
+{
+    uint32_t n = 0;
+    for (uint32_t i : items) n = std::max(n, i);
+    return n;
+}
+
+WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_width, uint32_t slots)
 {
     WavePlan plan;
     uint32_t max_spp = 0;
     for (uint32_t v = 0; v < view_count; ++v) max_spp = std::max(max_spp, views[v].params.spp);
     const uint32_t bh = 32u / block_width;
-    for (uint32_t s = 0; s < max_spp; ++s) {
-        std::vector<uint32_t> ids, bases;
+    for (uint32_t s = 0; s < max_spp;) {
+        // The views that have sample s, their items, and how many sample indices they all have left.
+        std::vector<uint32_t> ids, sizes;
         uint64_t items = 0;
-        uint32_t bounces = 0;
+        uint32_t bounces = 0, left = max_spp - s;
         for (uint32_t v = 0; v < view_count; ++v) {
             const TraceParams& p = views[v].params;
             if (p.spp <= s) continue;
-            ids.push_back(v);
-            bases.push_back((uint32_t)items);
             const uint64_t bx = (p.width + block_width - 1) / block_width, by = (p.height + bh - 1) / bh;
+            ids.push_back(v);
+            sizes.push_back((uint32_t)(32ull * bx * by));
             items += 32ull * bx * by;
             bounces = std::max(bounces, p.bounce_count);
+            left = std::min(left, p.spp - s);
         }
+        const uint32_t samples = items ? (uint32_t)std::min<uint64_t>(left, std::max<uint64_t>(slots / items, 1)) : 1u;
         plan.offset.push_back((uint32_t)plan.table.size());
-        plan.views.push_back((uint32_t)ids.size());
-        plan.items.push_back((uint32_t)std::min<uint64_t>(items, 0xFFFFFFFFull));
+        plan.entries.push_back((uint32_t)ids.size() * samples);
+        plan.samples.push_back(samples);
+        plan.items.push_back((uint32_t)std::min<uint64_t>(items * samples, 0xFFFFFFFFull));
         plan.bounces.push_back(bounces);
-        plan.table.insert(plan.table.end(), ids.begin(), ids.end());
-        plan.table.insert(plan.table.end(), bases.begin(), bases.end());
+        for (uint32_t k = 0; k < samples; ++k)
+            for (uint32_t id : ids) plan.table.push_back(id | ((s + k) << 16));
+        uint64_t base = 0;
+        for (uint32_t k = 0; k < samples; ++k)
+            for (uint32_t size : sizes) {
+                plan.table.push_back((uint32_t)base);
+                base += size;
+            }
+        s += samples;
     }
     return plan;
 }
@@ -617,12 +687,15 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
     }
     uint32_t count = 0;
     for (size_t s = 0; s < plan.items.size(); ++s) {
+        // Several sample indices: the whole wave in one sub-wave, then the samples' sums.
+        const bool resolve = plan.samples[s] > 1;
+        if (resolve && plan.items[s] > b.capacity) return cudaErrorInvalidValue;
         for (uint32_t first = 0; first < plan.items[s]; first += b.capacity) {
             const uint32_t n = std::min(b.capacity, plan.items[s] - first);
             WaveGen g;
             g.table = d_table + plan.offset[s];
-            g.n_views = plan.views[s];
-            g.sample = (uint32_t)s;
+            g.entries = plan.entries[s];
+            g.samples = plan.samples[s];
             g.first_item = first;
             g.count = n;
             g.block_width = block_width;
@@ -638,10 +711,17 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
                 if (entities) wave_trace_kernel<true, true><<<ray_grid, kWaveThreads, 0, stream>>>(d_views, b, parity);
                 else wave_trace_kernel<false, kMinBlocks == 8><<<ray_grid, kWaveThreads, 0, stream>>>(d_views, b, parity);
                 if (entities)
-                    wave_shade_kernel<kMode, kMinBlocks, true><<<shade_grid, kWaveThreads, 0, stream>>>(d_views, b, parity, adj);
+                    wave_shade_kernel<kMode, kMinBlocks, true><<<shade_grid, kWaveThreads, 0, stream>>>(d_views, b, parity, adj,
+                                                                                                       resolve);
                 else
-                    wave_shade_kernel<kMode, kMinBlocks, false><<<shade_grid, kWaveThreads, 0, stream>>>(d_views, b, parity, adj);
+                    wave_shade_kernel<kMode, kMinBlocks, false><<<shade_grid, kWaveThreads, 0, stream>>>(d_views, b, parity, adj,
+                                                                                                       resolve);
                 count += 2;
+            }
+            if (resolve && kMode != kShadeReplay) {
+                wave_resolve_kernel<<<(n / g.samples + kWaveThreads - 1) / kWaveThreads, kWaveThreads, 0, stream>>>(d_views, g,
+                                                                                                                 b);
+                ++count;
             }
             CX_TRY(cudaGetLastError());
         }
