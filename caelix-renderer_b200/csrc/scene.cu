@@ -131,14 +131,28 @@ __global__ void hash_place_kernel(const uint32_t* __restrict__ running_max, cons
     atomicMax(max_probe, pos - home_sorted[k]);
 }
 
-__global__ void bitmap_kernel(const int32_t* __restrict__ keys, uint32_t n, int32_t ox, int32_t oy, int32_t oz,
-                              uint32_t gx, uint32_t gy, uint32_t* __restrict__ bitmap)
+// The bitmap and the cell table (both zero before): the keys are in increasing linear brick index, so
+// the first brick of a 32-cell word gathers the word from the keys that follow (at most 31).
+__global__ void cell_table_kernel(const int32_t* __restrict__ keys, uint32_t n, int32_t ox, int32_t oy, int32_t oz,
+                                  uint32_t gx, uint32_t gy, uint32_t* __restrict__ bitmap, uint2* __restrict__ cells)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint64_t c = (uint64_t)(uint32_t)(keys[3 * i] - ox) +
-                       gx * ((uint64_t)(uint32_t)(keys[3 * i + 1] - oy) + (uint64_t)gy * (uint32_t)(keys[3 * i + 2] - oz));
-    atomicOr(bitmap + (c >> 5), 1u << (c & 31));
+    const auto index = [&](uint32_t j) {
+        return (uint64_t)(uint32_t)(keys[3ull * j] - ox) +
+               gx * ((uint64_t)(uint32_t)(keys[3ull * j + 1] - oy) + (uint64_t)gy * (uint32_t)(keys[3ull * j + 2] - oz));
+    };
+    const uint64_t c = index(i);
+    const uint64_t word = c >> 5;
+    if (i > 0 && (index(i - 1) >> 5) == word) return;
+    uint32_t bits = 1u << (c & 31);
+    for (uint32_t j = i + 1; j < n; ++j) {
+        const uint64_t d = index(j);
+        if ((d >> 5) != word) break;
+        bits |= 1u << (d & 31);
+    }
+    bitmap[word] = bits;
+    cells[word] = make_uint2(bits, i);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -937,10 +951,7 @@ SceneView scene_view(const DeviceScene& s)
     v.group_shift = s.group_shift;
     v.brick_count = s.brick_count;
     v.records = s.records;
-    v.hash_slots = s.hash_slots;
-    v.hash_capacity = s.hash_capacity;
-    v.hash_max_probe = s.hash_max_probe;
-    v.bitmap = s.bitmap;
+    v.cells = s.cells;
     v.power = s.power;
     v.materials = s.materials;
     v.light_codes = s.light_codes;
@@ -1047,7 +1058,7 @@ static BuildScratch build_scratch(const DeviceScene& s)
 void scene_release(DeviceScene& s)
 {
     void* ptrs[] = {s.keys,          s.voxels,       s.power,        s.records,       s.hash_slots,
-                    s.bitmap,        s.heap,         s.group_rows,    s.frames,
+                    s.bitmap,        s.cells,        s.heap,         s.group_rows,    s.frames,
                     s.light_headers, s.light_group,  s.light_entry,  s.light_brick,   s.scratch,
                     s.tree_memory,   s.status,       s.heap_prev,    s.unit_of_brick, s.unit_of_brick_prev,
                     s.group_gen,     s.group_flag};
@@ -1128,13 +1139,15 @@ cudaError_t scene_build_device(DeviceScene& s, const int32_t origin[3], const ui
         hash_place_kernel<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(tmp2, home, order, lo, hi, n, s.hash_slots,
                                                                             d_max_probe);
     }
-    // Bitmap.
+    // Bitmap and cell table.
     const uint64_t cells = (uint64_t)grid[0] * grid[1] * grid[2];
     CX_TRY(alloc(s.bitmap, s.capacity.bitmap, (cells + 31) / 32));
     CX_TRY(cudaMemsetAsync(s.bitmap, 0, 4 * ((cells + 31) / 32), stream));
+    CX_TRY(alloc(s.cells, s.capacity.cells, (cells + 31) / 32));
+    CX_TRY(cudaMemsetAsync(s.cells, 0, 8 * ((cells + 31) / 32), stream));
     if (n > 0)
-        bitmap_kernel<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(s.keys, n, origin[0], origin[1], origin[2],
-                                                                         grid[0], grid[1], s.bitmap);
+        cell_table_kernel<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(s.keys, n, origin[0], origin[1], origin[2],
+                                                                             grid[0], grid[1], s.bitmap, s.cells);
     CX_TRY(cudaMemcpyAsync(&s.hash_max_probe, d_max_probe, 4, cudaMemcpyDeviceToHost, stream));
     CX_TRY(cudaStreamSynchronize(stream));
 

@@ -65,10 +65,7 @@ struct SceneView
     int32_t origin[3];    // brick key of grid cell 0 (a multiple of the group edge)
     Encoding enc;
     const uint32_t* records;  // [brick_count][kRecordWords]
-    const uint4* hash_slots;  // key_lo, key_hi, record, 0
-    uint32_t hash_capacity;
-    uint32_t hash_max_probe;
-    const uint32_t* bitmap;  // brick occupancy by linear brick index
+    const uint2* cells;  // the cell table: per 32 linear brick indices the occupancy word and its first record
     const float* power;      // per-brick emitter power (a factor of the material emission)
     const float4* materials;  // [kMaterialCodes][2]: albedo, emission
     const uint32_t* light_codes;  // [kLightCodeWords]: the light code set
@@ -148,6 +145,7 @@ struct DeviceScene
     uint32_t* records = nullptr;
     uint4* hash_slots = nullptr;
     uint32_t* bitmap = nullptr;
+    uint2* cells = nullptr;  // the bitmap's words, each with the record of its first brick (cell_table_kernel)
     uint32_t* heap = nullptr;
     uint32_t* group_rows = nullptr;
     GroupFrame* frames = nullptr;
@@ -186,7 +184,7 @@ struct DeviceScene
     // Element capacities of the buffers above: a rebuild reallocates a buffer only to grow it.
     struct
     {
-        uint64_t keys, voxels, power, scratch, hash_slots, bitmap, records, group_rows, light_headers,
+        uint64_t keys, voxels, power, scratch, hash_slots, bitmap, cells, records, group_rows, light_headers,
             light_group, light_entry, light_brick, frames, heap, heap_prev, unit_of_brick, unit_of_brick_prev, group_gen,
             group_flag;
     } capacity{};
