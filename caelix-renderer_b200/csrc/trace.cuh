@@ -51,10 +51,11 @@ cudaError_t adjoint_launch(const SceneView& s, const TraceParams& p, const float
 // Paths live in HBM (structure of arrays, one slot per path); a wave is every pixel of one or more
 // consecutive sample indices of the views that have them (WavePlan), a wave of one sample index
 // split into sub-waves of at most `capacity` slots. Per bounce
-// two kernels run over compacted queues: wave_trace_kernel traces every queued ray (extension
-// and shadow rays alike, one DDA code path) and wave_shade_kernel advances every live path by
-// one vertex (shadow result, emission and MIS, albedo, light-tree NEE, Russian roulette),
-// queueing its next rays. Each kernel is small, and its warps start full.
+// three kernels run over compacted queues: wave_trace_kernel traces every queued ray (extension
+// and shadow rays alike, one DDA code path), wave_shade_kernel advances every live path by one
+// vertex (shadow result, emission, albedo, Russian roulette) and queues its extension ray and its
+// light-tree work, and wave_light_kernel does that work: the light draws (queueing the shadow rays)
+// and the MIS weights of lamp hits. Each kernel is small, and its warps start full.
 
 struct WaveView
 {
@@ -74,20 +75,24 @@ struct WaveBuffers
     uint32_t* flags = nullptr;
     uint32_t* rng = nullptr;
     uint32_t* light_rng = nullptr;
-    float4* org = nullptr;
-    float4* dir = nullptr;
-    float4* throughput = nullptr;
+    // The segment of a stage's parity (wave_shade_kernel writes the next one's; wave_light_kernel
+    // reads both): origin (the shadow ray's too), direction, throughput, the normal it left.
+    float4* org[2] = {nullptr, nullptr};
+    float4* dir[2] = {nullptr, nullptr};
+    float4* throughput[2] = {nullptr, nullptr};
+    float4* seg_n[2] = {nullptr, nullptr};
     float4* radiance = nullptr;
-    float4* seg_n = nullptr;
     float4* a0 = nullptr;    // primary albedo
     float4* e0 = nullptr;    // primary emission
     float4* sdir = nullptr;  // pending shadow ray: direction, t_max
-    float4* sadd = nullptr;  // pending shadow contribution
+    float4* sadd = nullptr;  // a light draw's vertex throughput, then the pending shadow contribution
     uint4* hit = nullptr;    // t bits, attrib (0 = miss), record, group
     uint32_t* occluded = nullptr;
     uint32_t* rayq[2] = {nullptr, nullptr};   // 2 * capacity entries: slot | kind << 30
     uint32_t* pathq[2] = {nullptr, nullptr};  // capacity entries
-    uint32_t* counts = nullptr;               // [parity][2]: rays, paths; then the trace fetch counters
+    uint32_t* neeq = nullptr;                 // capacity entries: slots that draw a light
+    uint32_t* lampq = nullptr;                // capacity entries: slots whose hit is a lamp (bit 31: the path ends there)
+    uint32_t* counts = nullptr;               // queue lengths and fetch counters (wave.cu)
     // The adjoint's per-slot state (wave_adjoint): dL/dR of the sample, its radiance R, the power
     // gradient of a pending NEE lamp (brick, value; applied if its shadow ray is unoccluded).
     float4* adj_g = nullptr;

@@ -1231,14 +1231,12 @@ __device__ __noinline__ float lamp_hit_weight(const SceneView& s, uint32_t segme
     return mis_weight(p_area, seg_n, dir, h.t, cos_l, false);
 }
 
-// The vertex of a hit: its material (the scene's table; an entity's bricks share it), its emission
-// (the table's times the brick's power) and the Lambertian bounce.
+// The material of a hit (the scene's table; an entity's bricks share it): its albedo, its emission
+// without the brick's power (me) and with it (emission).
 template <bool kEntities = true>
-__device__ __forceinline__ void shade(const SceneView& s, const Hit& h, const float ray_o[3], const float ray_d[3],
-                                      uint32_t& rng, float albedo[3], float emission[3], float origin[3], float dir[3])
+__device__ __forceinline__ void hit_emission(const SceneView& s, const Hit& h, float albedo[3], float me[3], float emission[3])
 {
-    const uint32_t block = (h.attrib >> 16) & 0xFFFFu;
-    material_of(s, block, albedo, emission);
+    material_of(s, (h.attrib >> 16) & 0xFFFFu, albedo, me);
     float P;
     if (kEntities && (h.attrib & kEntityHit)) {  // an entity brick's power
         const float* pw = s.entities[h.group >> kEntityShift].scene.power;
@@ -1247,7 +1245,16 @@ __device__ __forceinline__ void shade(const SceneView& s, const Hit& h, const fl
         P = __ldg(s.power + h.record);
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) emission[c] *= P;
+    for (int c = 0; c < 3; ++c) emission[c] = me[c] * P;
+}
+
+// The vertex of a hit: its material and emission, and the Lambertian bounce.
+template <bool kEntities = true>
+__device__ __forceinline__ void shade(const SceneView& s, const Hit& h, const float ray_o[3], const float ray_d[3],
+                                      uint32_t& rng, float albedo[3], float emission[3], float origin[3], float dir[3])
+{
+    float me[3];
+    hit_emission<kEntities>(s, h, albedo, me, emission);
     (void)random01(rng);  // the lobe draw (specular chance 0)
     float u[3];
     random_unit_vector(rng, u);
