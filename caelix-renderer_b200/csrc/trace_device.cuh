@@ -731,6 +731,21 @@ __device__ __forceinline__ void node_slot(const LightBvhNode* nd, uint32_t s, Su
     }
 }
 
+// Slots 2p and 2p + 1 of a node, in nine loads of 8 and 16 bytes (a slot by itself takes twelve).
+__device__ __forceinline__ void node_slot_pair(const LightBvhNode* nd, uint32_t p, Summary& a, Summary& b)
+{
+    const float4* f = reinterpret_cast<const float4*>(nd->child_face[2 * p]);
+    const float4 f0 = __ldg(f), f1 = __ldg(f + 1), f2 = __ldg(f + 2);
+    const float2* l = reinterpret_cast<const float2*>(nd->child_lo[2 * p]);
+    const float2 l0 = __ldg(l), l1 = __ldg(l + 1), l2 = __ldg(l + 2);
+    const float2* h = reinterpret_cast<const float2*>(nd->child_hi[2 * p]);
+    const float2 h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+    a.face[0] = f0.x, a.face[1] = f0.y, a.face[2] = f0.z, a.face[3] = f0.w, a.face[4] = f1.x, a.face[5] = f1.y;
+    b.face[0] = f1.z, b.face[1] = f1.w, b.face[2] = f2.x, b.face[3] = f2.y, b.face[4] = f2.z, b.face[5] = f2.w;
+    a.lo[0] = l0.x, a.lo[1] = l0.y, a.lo[2] = l1.x, b.lo[0] = l1.y, b.lo[1] = l2.x, b.lo[2] = l2.y;
+    a.hi[0] = h0.x, a.hi[1] = h0.y, a.hi[2] = h1.x, b.hi[0] = h1.y, b.hi[1] = h2.x, b.hi[2] = h2.y;
+}
+
 // Tree 0 is the world's tree; tree 1 the entities' (none without entity lights).
 __device__ __forceinline__ void tree_summary(const SceneView& s, uint32_t k, Summary& out, uint32_t& root)
 {
@@ -787,18 +802,27 @@ __device__ float slot_probability(const LightBvhNode* nd, const float x[3], cons
     const uint4 ch = __ldg(reinterpret_cast<const uint4*>(nd->child));
     if (child_count(ch) == 1) return 1.0f;
     float sum_i = 0.0f, sum_p = 0.0f, imp_t = 0.0f, pow_t = 0.0f;
-    for (uint32_t q = 0; q < 4; ++q) {
-        Summary sm;
-        node_slot(nd, q, sm);
-        const float imp = importance(x, n, sm.lo, sm.hi, sm.face);
-        const float pw = power6(sm.face);
-        if (__ldg(&nd->child[q]) != kNone) {
-            sum_i += imp > 0.0f ? imp : 0.0f;
-            sum_p += pw > 0.0f ? pw : 0.0f;
+    for (uint32_t p = 0; p < 2; ++p) {
+        Summary sm[2];
+        node_slot_pair(nd, p, sm[0], sm[1]);
+        float imp[2], pw[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            imp[i] = importance(x, n, sm[i].lo, sm[i].hi, sm[i].face);
+            pw[i] = power6(sm[i].face);
         }
-        if (q == slot) {
-            imp_t = imp;
-            pow_t = pw;
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t q = 2 * p + i;
+            const uint32_t c = p ? (i ? ch.w : ch.z) : (i ? ch.y : ch.x);
+            if (c != kNone) {
+                sum_i += imp[i] > 0.0f ? imp[i] : 0.0f;
+                sum_p += pw[i] > 0.0f ? pw[i] : 0.0f;
+            }
+            if (q == slot) {
+                imp_t = imp[i];
+                pow_t = pw[i];
+            }
         }
     }
     return pick_probability(sum_i, sum_p, imp_t, pow_t);
@@ -823,6 +847,103 @@ __device__ __noinline__ float leaf_probability(const SceneView& s, const SceneVi
         slot = up.y;
     }
     return 0.0f;
+}
+
+// The importances and powers of the four child slots of a node for a draw that four lanes share: each
+// lane evaluates its slot (lane & 3), then has all four. `busy` lanes only (the others get zeros); all
+// lanes of the warp call. Returns the slots that have a child (4 bits).
+struct QuadSlots
+{
+    float imp[4], pw;  // pw: this lane's slot's
+    uint32_t child;    // this lane's slot's
+};
+__device__ __forceinline__ uint32_t quad_slots(const LightBvhNode* nd, bool busy, const float x[3], const float n[3],
+                                               QuadSlots& o)
+{
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
+    float imp = 0.0f;
+    o.pw = 0.0f;
+    o.child = kNone;
+    if (busy) {
+        Summary sm;
+        const float2* f = reinterpret_cast<const float2*>(nd->child_face[q]);
+        const float2 f0 = __ldg(f), f1 = __ldg(f + 1), f2 = __ldg(f + 2);
+        sm.face[0] = f0.x;
+        sm.face[1] = f0.y;
+        sm.face[2] = f1.x;
+        sm.face[3] = f1.y;
+        sm.face[4] = f2.x;
+        sm.face[5] = f2.y;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            sm.lo[k] = __ldg(&nd->child_lo[q][k]);
+            sm.hi[k] = __ldg(&nd->child_hi[q][k]);
+        }
+        o.child = __ldg(&nd->child[q]);
+        imp = importance(x, n, sm.lo, sm.hi, sm.face);
+        o.pw = power6(sm.face);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o.imp[i] = __shfl_sync(0xFFFFFFFFu, imp, i, 4);
+    return (__ballot_sync(0xFFFFFFFFu, o.child != kNone) >> (lane & ~3u)) & 0xFu;
+}
+
+// The slot picks of leaf_probability (without the tree's) with four lanes per lamp hit (lane & 3: the
+// child slot), in the serial walk's order. `busy` is the same in the four lanes; all lanes call.
+__device__ __forceinline__ float leaf_walk_quad(const SceneView* L, uint32_t leaf, bool busy, const float x[3],
+                                                const float n[3])
+{
+    uint32_t node = 0, slot = 0;
+    float probability = 0.0f;
+    if (busy) {
+        const uint32_t parent = __ldg(&L->header->root) == kNone ? kNone : __ldg(&L->leaves[leaf].parent);
+        if (parent == kNone) {
+            busy = false;
+        } else {
+            node = parent >> kParentSlotBits;
+            slot = parent & kParentSlotMask;
+            probability = 1.0f;
+        }
+    }
+    for (uint32_t depth = 0; __any_sync(0xFFFFFFFFu, busy); ++depth) {
+        if (depth == 64) {
+            if (busy) probability = 0.0f;
+            break;
+        }
+        const LightBvhNode* nd = busy ? L->nodes + node : nullptr;
+        QuadSlots o;
+        const uint32_t has = quad_slots(nd, busy, x, n, o);
+        const bool many = busy && __popc(has) != 1;
+        float sum = 0.0f, own = 0.0f;
+        if (many) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                if ((has >> i) & 1u) sum += o.imp[i] > 0.0f ? o.imp[i] : 0.0f;
+                if (i == slot) own = o.imp[i];
+            }
+        }
+        const bool by_power = many && !(sum > 0.0f);
+        float sum_p = 0.0f, own_p = 0.0f;
+        if (__any_sync(0xFFFFFFFFu, by_power)) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const float pw = __shfl_sync(0xFFFFFFFFu, o.pw, i, 4);
+                if ((has >> i) & 1u) sum_p += pw > 0.0f ? pw : 0.0f;
+                if (i == slot) own_p = pw;
+            }
+        }
+        if (busy) {
+            if (many) probability *= pick_probability(sum, sum_p, own, own_p);
+            const uint2 up = __ldg(reinterpret_cast<const uint2*>(&nd->parent));
+            if (up.x == kNone) {
+                busy = false;
+            } else {
+                node = up.x;
+                slot = up.y;
+            }
+        }
+    }
+    return probability;
 }
 
 __device__ float family_weights(const SceneView& s, uint32_t group, const uint32_t* rec, const float x[3], float w[6])
@@ -879,37 +1000,46 @@ struct LightPoint
     uint32_t tree;  // 0: the world's light set, 1: the entities' (SceneView::dyn)
 };
 
-// kEntities: the scene may have a second (entity) light tree; without it only tree 0 is
-// evaluated and tree 1's draw is consumed (the same results for a scene without entity lights).
-template <bool kEntities = true>
-__device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3], const float n[3], uint32_t rng, LightPoint& p)
+// A light draw, in three parts: the tree, the walk down its 4-wide nodes to a leaf (a light brick),
+// the point on the brick.
+struct LightDraw
 {
-    float pdf_brick = 1.0f;
-    // The tree (one draw per tree; an empty tree's importance and power are never positive, so
-    // it only consumes its draw).
-    uint32_t root, k;
-    {
-        Pick pk = {0, 0, 0, 0, kNone, kNone};
-        uint32_t roots[2] = {kNone, kNone};
+    uint32_t rng;
+    uint32_t tree;  // 0: the world's, 1: the entities'
+    uint32_t root;  // of that tree
+    float pdf;      // of the choices so far
+};
+
+// The tree (one draw per tree; an empty tree's importance and power are never positive, so it only
+// consumes its draw). kEntities: the scene may have a second (entity) light tree; without it only
+// tree 0 is evaluated and tree 1's draw is consumed (the same results for a scene without entity
+// lights). False: no light is drawn.
+template <bool kEntities = true>
+__device__ __forceinline__ bool light_tree_pick(const SceneView& s, const float x[3], const float n[3], LightDraw& w)
+{
+    Pick pk = {0, 0, 0, 0, kNone, kNone};
+    uint32_t roots[2] = {kNone, kNone};
 #pragma unroll
-        for (uint32_t t = 0; t < 2; ++t) {
-            Summary sm;
-            if (kEntities || t == 0) tree_summary(s, t, sm, roots[t]);
-            const float u = lt_random_float(rng);
-            if (roots[t] != kNone) pick_add(pk, importance(x, n, sm.lo, sm.hi, sm.face), power6(sm.face), t, u);
-        }
-        float prob;
-        k = pick_end(pk, prob);
-        if (k == kNone) return false;
-        pdf_brick *= prob;
-        root = roots[k];
+    for (uint32_t t = 0; t < 2; ++t) {
+        Summary sm;
+        if (kEntities || t == 0) tree_summary(s, t, sm, roots[t]);
+        const float u = lt_random_float(w.rng);
+        if (roots[t] != kNone) pick_add(pk, importance(x, n, sm.lo, sm.hi, sm.face), power6(sm.face), t, u);
     }
-    const SceneView& L = (kEntities && k != 0) ? *s.dyn : s;
-    p.tree = k;
-    // Down the 4-wide nodes. Every slot's importance is computed by every lane (empty slots
-    // hold zero summaries and are skipped by the pick), so the lanes stay converged.
-    uint32_t leaf = kNone;
-    uint32_t node = root;
+    float prob;
+    w.tree = pick_end(pk, prob);
+    if (w.tree == kNone) return false;
+    w.pdf = 1.0f * prob;
+    w.root = roots[w.tree];
+    return true;
+}
+
+// Down the 4-wide nodes, one thread per draw: the leaf, or kNone. Every slot's importance is computed
+// by every lane (empty slots hold zero summaries and are skipped by the pick), so the lanes stay
+// converged.
+__device__ __forceinline__ uint32_t light_walk(const SceneView& L, const float x[3], const float n[3], LightDraw& w)
+{
+    uint32_t node = w.root;
     for (uint32_t depth = 0; depth < 64; ++depth) {
         const LightBvhNode* nd = L.nodes + node;
         const uint4 ch = __ldg(reinterpret_cast<const uint4*>(nd->child));
@@ -918,24 +1048,103 @@ __device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3
             chosen = ch.x;
         } else {
             Pick pk = {0, 0, 0, 0, kNone, kNone};
-            for (uint32_t q = 0; q < 4; ++q) {
-                Summary sm;
-                node_slot(nd, q, sm);
-                const float imp = importance(x, n, sm.lo, sm.hi, sm.face);
-                if (__ldg(&nd->child[q]) != kNone) pick_add(pk, imp, power6(sm.face), q, lt_random_float(rng));
+            for (uint32_t p = 0; p < 2; ++p) {
+                Summary a, b;
+                node_slot_pair(nd, p, a, b);
+                const float ia = importance(x, n, a.lo, a.hi, a.face);
+                const float ib = importance(x, n, b.lo, b.hi, b.face);
+                if ((p ? ch.z : ch.x) != kNone) pick_add(pk, ia, power6(a.face), 2 * p, lt_random_float(w.rng));
+                if ((p ? ch.w : ch.y) != kNone) pick_add(pk, ib, power6(b.face), 2 * p + 1, lt_random_float(w.rng));
             }
             float prob;
             const uint32_t q = pick_end(pk, prob);
-            if (q == kNone) return false;
-            pdf_brick *= prob;
+            if (q == kNone) return kNone;
+            w.pdf *= prob;
             chosen = __ldg(&nd->child[q]);
         }
-        if (chosen & kChildLeafBit) {
-            leaf = chosen & ~kChildLeafBit;
-            break;
-        }
+        if (chosen & kChildLeafBit) return chosen & ~kChildLeafBit;
         node = chosen;
     }
+    return kNone;
+}
+
+// light_walk with four lanes per draw (lane & 3: the child slot): the picks are those of the serial
+// walk, in slot order from the same random numbers, computed by each of the four lanes. `busy` is the
+// same in the four lanes; all lanes of the warp call.
+__device__ __forceinline__ uint32_t light_walk_quad(const LightBvhNode* nodes, bool busy, const float x[3], const float n[3],
+                                                    LightDraw& w)
+{
+    uint32_t node = w.root, leaf = kNone;
+    for (uint32_t depth = 0; depth < 64 && __any_sync(0xFFFFFFFFu, busy); ++depth) {
+        QuadSlots o;
+        const uint32_t has = quad_slots(nodes + node, busy, x, n, o);
+        uint32_t q = 0;
+        float prob = 1.0f;
+        float u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float sum = 0.0f;
+        if (busy && __popc(has) != 1) {
+            float weight = 0.0f;
+            q = kNone;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                if (!((has >> i) & 1u)) continue;
+                u[i] = lt_random_float(w.rng);
+                if (o.imp[i] > 0.0f) {
+                    sum += o.imp[i];
+                    if (u[i] * sum < o.imp[i]) {
+                        weight = o.imp[i];
+                        q = i;
+                    }
+                }
+            }
+            prob = weight / sum;
+        }
+        // No slot of positive importance: by power (pick_end).
+        const bool by_power = busy && __popc(has) != 1 && !(sum > 0.0f);
+        if (__any_sync(0xFFFFFFFFu, by_power)) {
+            float sum_p = 0.0f, weight_p = 0.0f;
+            uint32_t q_p = kNone;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const float pw = __shfl_sync(0xFFFFFFFFu, o.pw, i, 4);
+                if (((has >> i) & 1u) && pw > 0.0f) {
+                    sum_p += pw;
+                    if (u[i] * sum_p < pw) {
+                        weight_p = pw;
+                        q_p = i;
+                    }
+                }
+            }
+            if (by_power) {
+                prob = sum_p > 0.0f ? weight_p / sum_p : 0.0f;
+                q = sum_p > 0.0f ? q_p : kNone;
+            }
+        }
+        const uint32_t chosen = __shfl_sync(0xFFFFFFFFu, o.child, q == kNone ? 0u : q, 4);
+        if (busy) {
+            if (q == kNone) {
+                busy = false;
+            } else {
+                if (__popc(has) != 1) w.pdf *= prob;
+                if (chosen & kChildLeafBit) {
+                    leaf = chosen & ~kChildLeafBit;
+                    busy = false;
+                } else {
+                    node = chosen;
+                }
+            }
+        }
+    }
+    return leaf;
+}
+
+// The point on light brick `leaf` of the draw's tree (its light set L). False: no point.
+__device__ __forceinline__ bool light_point(const SceneView& L, const float x[3], const LightDraw& w, uint32_t leaf,
+                                            LightPoint& p)
+{
+    uint32_t rng = w.rng;
+    const float pdf_brick = w.pdf;
+    p.tree = w.tree;
     if (leaf == kNone) return false;
     const uint2 owner = __ldg(reinterpret_cast<const uint2*>(&L.leaves[leaf].group));
     const uint32_t group = owner.x, entry = owner.y;
@@ -945,17 +1154,17 @@ __device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3
     if (row.y == 0) return false;
     const uint32_t* block = L.heap + 4ull * row.x;
     const uint32_t* rec = block + 4ull * __ldg(block + 4 + 4 * entry + 2);
-    float w[6];
-    const float sum = family_weights(L, group, rec, x, w);
+    float fw[6];
+    const float sum = family_weights(L, group, rec, x, fw);
     if (sum <= 0.0f) return false;
     const float u = lt_random_float(rng) * sum;
     uint32_t f = kNone, last = 0;
     float cumulative = 0.0f;
 #pragma unroll
     for (uint32_t g = 0; g < 6; ++g) {
-        if (w[g] > 0.0f) {
+        if (fw[g] > 0.0f) {
             last = g;
-            cumulative += w[g];
+            cumulative += fw[g];
             if (f == kNone && u < cumulative) f = g;
         }
     }
@@ -970,7 +1179,7 @@ __device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3
         if (g < f) first += c;
         if (g == f) {
             count = c;
-            wf = w[g];
+            wf = fw[g];
         }
     }
     if (count == 0 || wf <= 0.0f) return false;
@@ -1005,6 +1214,18 @@ __device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3
     p.pdf = wf / sum / (float)count * pdf_brick;
     p.block = ent >> 16;
     return true;
+}
+
+// A whole draw by one thread.
+template <bool kEntities = true>
+__device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3], const float n[3], uint32_t rng, LightPoint& p)
+{
+    LightDraw w;
+    w.rng = rng;
+    if (!light_tree_pick<kEntities>(s, x, n, w)) return false;
+    const SceneView& L = (kEntities && w.tree != 0) ? *s.dyn : s;
+    const uint32_t leaf = light_walk(L, x, n, w);
+    return light_point(L, x, w, leaf, p);
 }
 
 // LightTreeFindLightFace (caelix_light_tree.hlsl:853-935): the face of a voxel whose material code
@@ -1088,20 +1309,18 @@ __device__ __noinline__ bool find_light_face(const SceneView& s, const float x[3
     return true;
 }
 
-// The draw probability of entry `entry` of group `group` of light set k (L).
-__device__ float brick_pdf(const SceneView& s, const SceneView& L, const float x[3], const float n[3], uint32_t group,
-                           uint32_t entry, uint32_t k)
+// The leaf of entry `entry` of group `group` of light set L, or kNone (its draw probability is 0).
+__device__ __forceinline__ uint32_t brick_leaf(const SceneView& L, uint32_t group, uint32_t entry)
 {
     const uint2 row = __ldg(reinterpret_cast<const uint2*>(L.group_rows + 8ull * group));
-    if (row.y == 0) return 0.0f;
+    if (row.y == 0) return kNone;
     const uint32_t* block = L.heap + 4ull * row.x;
-    if (entry >= __ldg(block)) return 0.0f;
+    if (entry >= __ldg(block)) return kNone;
     const uint32_t bvh_leaf = __ldg(block + 4 + 4 * entry + 3);
-    if (bvh_leaf == kNone) return 0.0f;
+    if (bvh_leaf == kNone) return kNone;
     const uint32_t leaf = bvh_leaf & 0x7FFFFFFFu;
     const uint2 owner = __ldg(reinterpret_cast<const uint2*>(&L.leaves[leaf].group));
-    if (owner.x != group || owner.y != entry) return 0.0f;
-    return leaf_probability(s, L, leaf, x, n, k);
+    return owner.x != group || owner.y != entry ? kNone : leaf;
 }
 
 // ---- integrator ----
@@ -1149,12 +1368,10 @@ __device__ __forceinline__ void material_of(const SceneView& s, uint32_t block, 
 }
 
 template <bool kEntities = true>
-__device__ __forceinline__ bool nee_prepare(const SceneView& s, const float x[3], const float n[3], uint32_t& light_rng,
-                                            ShadowRay& r)
+__device__ __forceinline__ bool nee_shadow_ray(const SceneView& s, const float x[3], const float n[3], const LightPoint& p,
+                                               ShadowRay& r)
 {
-    const uint32_t point_seed = random_u32(light_rng);
-    LightPoint p;
-    if (!light_sample<kEntities>(s, x, n, point_seed, p) || !(p.pdf > 0.0f)) return false;
+    if (!(p.pdf > 0.0f)) return false;
     const float d[3] = {p.position[0] - x[0], p.position[1] - x[1], p.position[2] - x[2]};
     const float d2 = dot3(d, d);
     const float dist = sqrtf(d2);
@@ -1197,17 +1414,35 @@ __device__ __forceinline__ bool nee_prepare(const SceneView& s, const float x[3]
     return true;
 }
 
-__device__ __noinline__ float lamp_hit_weight(const SceneView& s, uint32_t segment_light, const Hit& h, const float origin[3],
-                                 const float dir[3], const float seg_n[3])
+template <bool kEntities = true>
+__device__ __forceinline__ bool nee_prepare(const SceneView& s, const float x[3], const float n[3], uint32_t& light_rng,
+                                            ShadowRay& r)
 {
-    if (segment_light == 0u || h.t < kNearField) return 1.0f;
+    const uint32_t point_seed = random_u32(light_rng);
+    LightPoint p;
+    return light_sample<kEntities>(s, x, n, point_seed, p) && nee_shadow_ray<kEntities>(s, x, n, p, r);
+}
+
+// A lamp hit whose MIS weight needs the probability that the draw at the segment's origin had of it:
+// the light brick's leaf of the tree, and the part of the probability inside the brick.
+struct LampHit
+{
+    const SceneView* set;  // the light set of the tree
+    uint32_t tree;
+    uint32_t leaf;         // kNone: the brick is never drawn (probability 0)
+    float in_brick;
+};
+
+// False: the draw cannot reach this hit (its weight is 1).
+__device__ __forceinline__ bool lamp_lookup(const SceneView& s, const Hit& h, const float origin[3], LampHit& o)
+{
     // The light set of the hit: tree 0's for the world and static entities, the dynamic one for
     // dynamic entities (an entity's groups from its group base; the voxel from the entity-local
     // hit point and face normal).
     const uint32_t face = (uint32_t)(__ffs(h.attrib & 0x3Fu) - 1);
     const bool entity = (h.attrib & kEntityHit) != 0;
     const uint32_t tree = entity ? __ldg(&s.entities[h.group >> kEntityShift].tree) : 0u;
-    if (tree > 1u || (tree == 1u && !s.dyn)) return 1.0f;
+    if (tree > 1u || (tree == 1u && !s.dyn)) return false;
     const SceneView& L = tree == 1u ? *s.dyn : s;
     const uint32_t group = entity ? __ldg(&s.entities[h.group >> kEntityShift].group_base) + (h.group & kEntityGroupMask)
                                   : h.group;
@@ -1224,11 +1459,28 @@ __device__ __noinline__ float lamp_hit_weight(const SceneView& s, uint32_t segme
     }
     const uint32_t block = (h.attrib >> 16) & 0xFFFFu;
     uint32_t entry, leaf;
-    float in_brick;
-    if (!find_light_face(L, origin, group, vig, face, block, entry, leaf, in_brick) || leaf == kNone) return 1.0f;
+    if (!find_light_face(L, origin, group, vig, face, block, entry, leaf, o.in_brick) || leaf == kNone) return false;
+    o.set = &L;
+    o.tree = tree;
+    o.leaf = brick_leaf(L, group, entry);
+    return true;
+}
+
+__device__ __forceinline__ float lamp_weight(const Hit& h, const LampHit& l, float brick_probability, const float dir[3],
+                                             const float seg_n[3])
+{
     const float cos_l = -dot3(h.normal, dir);
-    const float p_area = brick_pdf(s, L, origin, seg_n, group, entry, tree) * in_brick;
-    return mis_weight(p_area, seg_n, dir, h.t, cos_l, false);
+    return mis_weight(brick_probability * l.in_brick, seg_n, dir, h.t, cos_l, false);
+}
+
+__device__ __noinline__ float lamp_hit_weight(const SceneView& s, uint32_t segment_light, const Hit& h, const float origin[3],
+                                 const float dir[3], const float seg_n[3])
+{
+    if (segment_light == 0u || h.t < kNearField) return 1.0f;
+    LampHit l;
+    if (!lamp_lookup(s, h, origin, l)) return 1.0f;
+    const float p = l.leaf == kNone ? 0.0f : leaf_probability(s, *l.set, l.leaf, origin, seg_n, l.tree);
+    return lamp_weight(h, l, p, dir, seg_n);
 }
 
 // The material of a hit (the scene's table; an entity's bricks share it): its albedo, its emission

@@ -572,6 +572,17 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     }
 }
 
+// Waves of at most this many paths do their light-tree work with four lanes per item.
+constexpr uint32_t kQuadPaths = 1u << 16;
+
+// The next chunk's index for the calling warp, from a fetch counter. Every lane calls.
+__device__ __forceinline__ uint32_t fetch_one(uint32_t* counter)
+{
+    uint32_t c = 0;
+    if ((threadIdx.x & 31u) == 0) c = atomicAdd(counter, 1u);
+    return __shfl_sync(0xFFFFFFFFu, c, 0);
+}
+
 // The light-tree work that the shade launch queued: the light draws (a vertex's NEE up to its shadow
 // ray, which is queued), then the lamp hits (the MIS weight of the hit against the draw of the vertex
 // before it, then its emission). In the shade kernel, where half of a warp's paths miss or end and
@@ -579,7 +590,13 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
 // 512, 1 spp 0.520 -> 0.496 ms; 333 x 251, 8 spp 1.11 -> 0.93; 1920 x 1080, 4 spp on 300 k bricks
 // 19.9 -> 14.3; the adjoint of 256 x 256, 8 spp over a world of lamps 3.24 -> 2.11. A frame of 14 k
 // paths, all launch latency, pays for the third launch per stage: 0.133 -> 0.145.
-template <int kMode, int kMinBlocks, bool kEntities>
+//
+// A warp takes 32 draws or 32 lamp hits, a lane each. kQuad: eight, and four lanes share an item's
+// walk through the tree, a child slot each: for waves of few paths, whose launches are chains of
+// dependent levels on a chip that is mostly idle. Measured, four lanes against one (1 spp, 4 bounces):
+// 200 x 150 0.287 against 0.305 ms, 256 x 256 on 20 k bricks 0.429 against 0.473, 400 x 300 0.376
+// against 0.381, 512 x 512 0.578 against 0.516 (there the chip is full, and four lanes repeat the pick).
+template <int kMode, int kMinBlocks, bool kEntities, bool kQuad>
 __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     wave_light_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj,
                       bool resolve)
@@ -594,26 +611,77 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     }
     const uint32_t draws = *(volatile uint32_t*)&b.counts[kCountNee];
     const uint32_t lamps = *(volatile uint32_t*)&b.counts[kCountLamp];
-    const uint32_t first_lamp = (draws + 31u) & ~31u;  // a chunk of 32 holds one kind
-    const uint32_t n = first_lamp + lamps;
+    constexpr uint32_t chunk = kQuad ? 8u : 32u;
+    const uint32_t draw_chunks = (draws + chunk - 1) / chunk;
+    const uint32_t chunks = draw_chunks + (lamps + chunk - 1) / chunk;
     const uint32_t out = parity ^ 1u;
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t base = fetch_chunk(&b.counts[kFetchLight]); base < n; base = fetch_chunk(&b.counts[kFetchLight])) {
-        const uint32_t i = base + lane;
-        if (base < first_lamp) {
-            bool shadow = false;
-            uint32_t slot = 0;
-            if (i < draws) {
-                slot = b.neeq[i];
-                const SceneView& S = views[b.vs[slot] & 0xFFFFu].scene;
+    uint32_t* const fetch = &b.counts[kFetchLight];
+    for (uint32_t c = fetch_one(fetch); c < chunks; c = fetch_one(fetch)) {
+        const bool draw = c < draw_chunks;
+        const uint32_t base = (draw ? c : c - draw_chunks) * chunk;
+        const uint32_t count = min(chunk, (draw ? draws : lamps) - base);
+        const bool mine = lane < count;
+        uint32_t slot = 0, entry = 0;
+        const SceneView* S = nullptr;
+        float x[3] = {0.0f, 0.0f, 0.0f}, nrm[3] = {0.0f, 0.0f, 0.0f};
+        bool walk = false;
+        const SceneView* set = nullptr;  // the light set the walk is in
+        if (draw) {
+            LightDraw w = {0u, 0u, 0u, 1.0f};
+            uint32_t light_rng = 0;
+            if (mine) {
+                slot = b.neeq[base + lane];
+                S = &views[b.vs[slot] & 0xFFFFu].scene;
                 const float4 o4 = b.org[out][slot];
                 const float4 n4 = b.seg_n[out][slot];
-                const float x[3] = {o4.x, o4.y, o4.z};
-                const float nrm[3] = {n4.x, n4.y, n4.z};
-                uint32_t light_rng = b.light_rng[slot];
-                ShadowRay r;
-                shadow = nee_prepare<kEntities>(S, x, nrm, light_rng, r);
+                x[0] = o4.x;
+                x[1] = o4.y;
+                x[2] = o4.z;
+                nrm[0] = n4.x;
+                nrm[1] = n4.y;
+                nrm[2] = n4.z;
+                light_rng = b.light_rng[slot];
+                w.rng = random_u32(light_rng);
                 b.light_rng[slot] = light_rng;
+                walk = light_tree_pick<kEntities>(*S, x, nrm, w);
+                set = (kEntities && w.tree == 1u) ? S->dyn : S;
+            }
+            uint32_t leaf = kNone;
+            if constexpr (!kQuad) {
+                if (walk) leaf = light_walk(*set, x, nrm, w);
+            } else {
+                const uint32_t from = lane >> 2;
+                float qx[3], qn[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    qx[k] = __shfl_sync(0xFFFFFFFFu, x[k], from);
+                    qn[k] = __shfl_sync(0xFFFFFFFFu, nrm[k], from);
+                }
+                LightDraw qw;
+                qw.rng = __shfl_sync(0xFFFFFFFFu, w.rng, from);
+                qw.root = __shfl_sync(0xFFFFFFFFu, w.root, from);
+                qw.pdf = __shfl_sync(0xFFFFFFFFu, w.pdf, from);
+                const bool busy = __shfl_sync(0xFFFFFFFFu, walk ? 1u : 0u, from) != 0u;
+                const uint64_t qset = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(set), from);
+                const LightBvhNode* nodes = busy ? reinterpret_cast<const SceneView*>(qset)->nodes : nullptr;
+                const uint32_t found = light_walk_quad(nodes, busy, qx, qn, qw);
+                // Back to the item's lane.
+                const uint32_t to = 4u * (lane & 7u);
+                const uint32_t l = __shfl_sync(0xFFFFFFFFu, found, to);
+                const uint32_t rng = __shfl_sync(0xFFFFFFFFu, qw.rng, to);
+                const float pdf = __shfl_sync(0xFFFFFFFFu, qw.pdf, to);
+                if (mine) {
+                    leaf = l;
+                    w.rng = rng;
+                    w.pdf = pdf;
+                }
+            }
+            bool shadow = false;
+            if (walk) {
+                LightPoint p;
+                ShadowRay r;
+                shadow = light_point(*set, x, w, leaf, p) && nee_shadow_ray<kEntities>(*S, x, nrm, p, r);
                 if (shadow) {
                     const float4 t4 = b.sadd[slot];
                     const float tp[3] = {t4.x, t4.y, t4.z};
@@ -638,43 +706,78 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
             }
             const uint32_t q = warp_append(&b.counts[2 * out], shadow ? 1u : 0u);
             if (shadow) b.rayq[out][q] = slot | (kKindShadow << 30);
-        } else if (i < n) {
-            const uint32_t entry = b.lampq[i - first_lamp];
-            const uint32_t slot = entry & ~kLampEnds;
-            const uint32_t vs = b.vs[slot];
-            const WaveView& V = views[vs & 0xFFFFu];
-            const SceneView& S = V.scene;
-            const float4 o4 = b.org[parity][slot];
-            const float4 d4 = b.dir[parity][slot];
-            const float4 n4 = b.seg_n[parity][slot];
-            const float4 t4 = b.throughput[parity][slot];
-            const float4 r4 = b.radiance[slot];
-            const float org[3] = {o4.x, o4.y, o4.z};
-            const float dir[3] = {d4.x, d4.y, d4.z};
-            const float seg_n[3] = {n4.x, n4.y, n4.z};
-            const float tp[3] = {t4.x, t4.y, t4.z};
-            float rad[3] = {r4.x, r4.y, r4.z};
-            const Hit h = unpack_hit<kEntities>(S, b.hit[slot], org, dir);
-            const float ew = lamp_hit_weight(S, 3u, h, org, dir, seg_n);
-            float al[3], me[3], em[3];
-            hit_emission<kEntities>(S, h, al, me, em);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) rad[k] += em[k] * (tp[k] * ew);
-            if (kMode == kShadeReplay) {
-                const float4 g4 = b.adj_g[slot];
-                const float4 s4 = b.adj_r[slot];
-                const float G[3] = {g4.x, g4.y, g4.z};
-                const float R[3] = {s4.x, s4.y, s4.z};
-                replay_vertex(S, adj, cache, h, G, R, rad, tp, ew, me, al);
+        } else {
+            Hit h;
+            LampHit lamp = {nullptr, 0u, kNone, 0.0f};
+            float dir[3] = {0.0f, 0.0f, 0.0f};
+            bool weighed = false;
+            uint32_t vs = 0;
+            if (mine) {
+                entry = b.lampq[base + lane];
+                slot = entry & ~kLampEnds;
+                vs = b.vs[slot];
+                S = &views[vs & 0xFFFFu].scene;
+                const float4 o4 = b.org[parity][slot];
+                const float4 d4 = b.dir[parity][slot];
+                const float4 n4 = b.seg_n[parity][slot];
+                x[0] = o4.x;
+                x[1] = o4.y;
+                x[2] = o4.z;
+                dir[0] = d4.x;
+                dir[1] = d4.y;
+                dir[2] = d4.z;
+                nrm[0] = n4.x;
+                nrm[1] = n4.y;
+                nrm[2] = n4.z;
+                h = unpack_hit<kEntities>(*S, b.hit[slot], x, dir);
+                weighed = lamp_lookup(*S, h, x, lamp);
+                walk = weighed && lamp.leaf != kNone;
             }
-            if (entry & kLampEnds) {
-                const float4 a4 = b.a0[slot];
-                const float4 e4 = b.e0[slot];
-                const float a0[3] = {a4.x, a4.y, a4.z};
-                const float e0[3] = {e4.x, e4.y, e4.z};
-                finish_path<kMode>(V, b, adj, slot, b.item[slot], vs >> 16, false, rad, e0, a0, resolve);
+            float probability = 0.0f;
+            if constexpr (!kQuad) {
+                if (walk) probability = leaf_probability(*S, *lamp.set, lamp.leaf, x, nrm, lamp.tree);
             } else {
-                b.radiance[slot] = make_float4(rad[0], rad[1], rad[2], 0.0f);
+                const uint32_t from = lane >> 2;
+                float qx[3], qn[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    qx[k] = __shfl_sync(0xFFFFFFFFu, x[k], from);
+                    qn[k] = __shfl_sync(0xFFFFFFFFu, nrm[k], from);
+                }
+                const uint32_t leaf = __shfl_sync(0xFFFFFFFFu, lamp.leaf, from);
+                const bool busy = __shfl_sync(0xFFFFFFFFu, walk ? 1u : 0u, from) != 0u;
+                const uint64_t qset = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(lamp.set), from);
+                const float found = leaf_walk_quad(reinterpret_cast<const SceneView*>(qset), leaf, busy, qx, qn);
+                probability = __shfl_sync(0xFFFFFFFFu, found, 4u * (lane & 7u));
+                if (walk) probability = probability * tree_probability(*S, x, nrm, lamp.tree);
+            }
+            if (mine) {
+                const float ew = weighed ? lamp_weight(h, lamp, probability, dir, nrm) : 1.0f;
+                const WaveView& V = views[vs & 0xFFFFu];
+                const float4 t4 = b.throughput[parity][slot];
+                const float4 r4 = b.radiance[slot];
+                const float tp[3] = {t4.x, t4.y, t4.z};
+                float rad[3] = {r4.x, r4.y, r4.z};
+                float al[3], me[3], em[3];
+                hit_emission<kEntities>(*S, h, al, me, em);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) rad[k] += em[k] * (tp[k] * ew);
+                if (kMode == kShadeReplay) {
+                    const float4 g4 = b.adj_g[slot];
+                    const float4 s4 = b.adj_r[slot];
+                    const float G[3] = {g4.x, g4.y, g4.z};
+                    const float R[3] = {s4.x, s4.y, s4.z};
+                    replay_vertex(*S, adj, cache, h, G, R, rad, tp, ew, me, al);
+                }
+                if (entry & kLampEnds) {
+                    const float4 a4 = b.a0[slot];
+                    const float4 e4 = b.e0[slot];
+                    const float a0[3] = {a4.x, a4.y, a4.z};
+                    const float e0[3] = {e4.x, e4.y, e4.z};
+                    finish_path<kMode>(V, b, adj, slot, b.item[slot], vs >> 16, false, rad, e0, a0, resolve);
+                } else {
+                    b.radiance[slot] = make_float4(rad[0], rad[1], rad[2], 0.0f);
+                }
             }
         }
     }
@@ -812,9 +915,9 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
                                                              kWaveThreads, 0));
         CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shade_blocks[1], wave_shade_kernel<kMode, kMinBlocks, true>,
                                                              kWaveThreads, 0));
-        CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&light_blocks[0], wave_light_kernel<kMode, kMinBlocks, false>,
+        CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&light_blocks[0], wave_light_kernel<kMode, kMinBlocks, false, false>,
                                                              kWaveThreads, 0));
-        CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&light_blocks[1], wave_light_kernel<kMode, kMinBlocks, true>,
+        CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&light_blocks[1], wave_light_kernel<kMode, kMinBlocks, true, false>,
                                                              kWaveThreads, 0));
         for (int k = 0; k < 2; ++k) {
             light_blocks[k] = std::max(light_blocks[k], 1);
@@ -846,14 +949,20 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
             // At most a light draw and a lamp hit per path; chunks of 32.
             const uint32_t light_grid = std::min<uint32_t>((2 * n + kWaveThreads - 1) / kWaveThreads,
                                                            sm_count * (uint32_t)light_blocks[entities ? 1 : 0]);
+            const bool quad = n <= kQuadPaths;
+            const uint32_t quad_grid = std::min<uint32_t>((8 * n + kWaveThreads - 1) / kWaveThreads, sm_count * 5);
             const auto stage = [&](auto with_entities, uint32_t parity) {
                 constexpr bool kEntities = decltype(with_entities)::value;
                 wave_trace_kernel<kEntities, kEntities || kMinBlocks == 8><<<ray_grid, kWaveThreads, 0, stream>>>(d_views, b,
                                                                                                           parity);
                 wave_shade_kernel<kMode, kMinBlocks, kEntities><<<shade_grid, kWaveThreads, 0, stream>>>(d_views, b, parity,
                                                                                                  adj, resolve);
-                wave_light_kernel<kMode, kMinBlocks, kEntities><<<light_grid, kWaveThreads, 0, stream>>>(d_views, b, parity,
-                                                                                                 adj, resolve);
+                if (quad)
+                    wave_light_kernel<kMode, 5, kEntities, true><<<quad_grid, kWaveThreads, 0, stream>>>(d_views, b, parity, adj,
+                                                                                                resolve);
+                else
+                    wave_light_kernel<kMode, kMinBlocks, kEntities, false><<<light_grid, kWaveThreads, 0, stream>>>(
+                        d_views, b, parity, adj, resolve);
             };
             for (uint32_t it = 0; it <= plan.bounces[s]; ++it) {
                 if (entities) stage(std::true_type{}, it & 1u);
