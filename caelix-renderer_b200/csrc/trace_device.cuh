@@ -1036,7 +1036,9 @@ __device__ __forceinline__ bool light_tree_pick(const SceneView& s, const float 
 
 // Down the 4-wide nodes, one thread per draw: the leaf, or kNone. Every slot's importance is computed
 // by every lane (empty slots hold zero summaries and are skipped by the pick), so the lanes stay
-// converged.
+// converged. kPairs: two slots at a time, from wide loads (the light kernel); the kernels that trace
+// and shade in one have no registers for it.
+template <bool kPairs>
 __device__ __forceinline__ uint32_t light_walk(const SceneView& L, const float x[3], const float n[3], LightDraw& w)
 {
     uint32_t node = w.root;
@@ -1048,13 +1050,22 @@ __device__ __forceinline__ uint32_t light_walk(const SceneView& L, const float x
             chosen = ch.x;
         } else {
             Pick pk = {0, 0, 0, 0, kNone, kNone};
-            for (uint32_t p = 0; p < 2; ++p) {
-                Summary a, b;
-                node_slot_pair(nd, p, a, b);
-                const float ia = importance(x, n, a.lo, a.hi, a.face);
-                const float ib = importance(x, n, b.lo, b.hi, b.face);
-                if ((p ? ch.z : ch.x) != kNone) pick_add(pk, ia, power6(a.face), 2 * p, lt_random_float(w.rng));
-                if ((p ? ch.w : ch.y) != kNone) pick_add(pk, ib, power6(b.face), 2 * p + 1, lt_random_float(w.rng));
+            if constexpr (kPairs) {
+                for (uint32_t p = 0; p < 2; ++p) {
+                    Summary a, b;
+                    node_slot_pair(nd, p, a, b);
+                    const float ia = importance(x, n, a.lo, a.hi, a.face);
+                    const float ib = importance(x, n, b.lo, b.hi, b.face);
+                    if ((p ? ch.z : ch.x) != kNone) pick_add(pk, ia, power6(a.face), 2 * p, lt_random_float(w.rng));
+                    if ((p ? ch.w : ch.y) != kNone) pick_add(pk, ib, power6(b.face), 2 * p + 1, lt_random_float(w.rng));
+                }
+            } else {
+                for (uint32_t q = 0; q < 4; ++q) {
+                    Summary sm;
+                    node_slot(nd, q, sm);
+                    const float imp = importance(x, n, sm.lo, sm.hi, sm.face);
+                    if (__ldg(&nd->child[q]) != kNone) pick_add(pk, imp, power6(sm.face), q, lt_random_float(w.rng));
+                }
             }
             float prob;
             const uint32_t q = pick_end(pk, prob);
@@ -1224,7 +1235,7 @@ __device__ __forceinline__ bool light_sample(const SceneView& s, const float x[3
     w.rng = rng;
     if (!light_tree_pick<kEntities>(s, x, n, w)) return false;
     const SceneView& L = (kEntities && w.tree != 0) ? *s.dyn : s;
-    const uint32_t leaf = light_walk(L, x, n, w);
+    const uint32_t leaf = light_walk<false>(L, x, n, w);
     return light_point(L, x, w, leaf, p);
 }
 

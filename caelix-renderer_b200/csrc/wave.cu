@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
             }
             uint32_t leaf = kNone;
             if constexpr (!kQuad) {
-                if (walk) leaf = light_walk(*set, x, nrm, w);
+                if (walk) leaf = light_walk<true>(*set, x, nrm, w);
             } else {
                 const uint32_t from = lane >> 2;
                 float qx[3], qn[3];

@@ -698,7 +698,11 @@ typedef struct CaelixBatchTuning
     uint32_t order;                /* 0 = views in the given order, 1 = the most pixel samples first */
     uint32_t kernel;               /* CAELIX_BATCH_PERSISTENT: one persistent launch traces every
                                       view; CAELIX_BATCH_WAVEFRONT: the wavefront kernels of
-                                      caelix_renderer_set_trace_mode over the paths of every view */
+                                      caelix_renderer_set_trace_mode over the paths of every view.
+                                      A batch whose tuning was neither set nor autotuned is traced
+                                      by the wavefront kernels in 8 x 4 blocks (every organisation
+                                      gives the same radiance; CaelixBatchStats::wavefront tells
+                                      the paths in flight) */
     uint32_t reserved;             /* must be 0 */
 } CaelixBatchTuning;
 #define CAELIX_BATCH_PERSISTENT 0u

@@ -96,3 +96,38 @@ def test_batch_of_unequal_samples(cuda_device):
     batch.close()
     r.close()
     scene.close()
+
+
+def test_untuned_batch_is_traced_by_the_wavefront_kernels(cuda_device):
+    """A batch that was never tuned runs the wavefront kernels; setting the reported tuning runs the
+    persistent kernel; both give the plain renders' radiance."""
+    import torch
+
+    import caelix_b200
+
+    vs = world()
+    scene = caelix_b200.Scene.from_voxel_scene(cuda_device, vs)
+    r = caelix_b200.Renderer(cuda_device, scene)
+    shapes = [(37, 21, 2), (8, 4, 1)]
+    outs = [torch.zeros(w * h * 3, device="cuda") for w, h, _ in shapes]
+    refs = [torch.zeros_like(o) for o in outs]
+    for i, (ref, (w, h, spp)) in enumerate(zip(refs, shapes)):
+        r.render(ref, w, h, vs.camera, bounces=3, seed=5 + i, spp=spp)
+    views = [(r, o, w, h, vs.camera, 3, 5 + i, spp) for i, (o, (w, h, spp)) in enumerate(zip(outs, shapes))]
+    batch = caelix_b200.Batch(cuda_device, views)
+    for tuned in (False, True):
+        if tuned:
+            assert batch.tuning().kernel == 0
+            batch.set_tuning()
+        for o in outs:
+            o.fill_(-1.0)
+        batch.run()
+        st = batch.stats()
+        # The second view has one sample only, so the views' samples do not join one wave.
+        paths = items(37, 21) + items(8, 4)
+        assert (st.wavefront == paths) == (not tuned)
+        for ref, o in zip(refs, outs):
+            assert torch.equal(ref, o)
+    batch.close()
+    r.close()
+    scene.close()
