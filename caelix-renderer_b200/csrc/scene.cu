@@ -946,6 +946,8 @@ SceneView scene_view(const DeviceScene& s)
         v.grid[k] = s.grid[k];
         v.groups[k] = s.groups[k];
         v.origin[k] = s.origin[k];
+        v.low[k] = (float)(8 * s.origin[k]);
+        v.high[k] = (float)(8 * (s.origin[k] + (int)s.grid[k]));
     }
     v.enc = encoding_of(s.encoding);
     v.group_shift = s.group_shift;

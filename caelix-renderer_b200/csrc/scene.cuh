@@ -63,6 +63,7 @@ struct SceneView
     uint32_t groups[3];
     uint32_t brick_count;
     int32_t origin[3];    // brick key of grid cell 0 (a multiple of the group edge)
+    float low[3], high[3];  // the grid's voxel box
     Encoding enc;
     const uint32_t* records;  // [brick_count][kRecordWords]
     const uint2* cells;  // the cell table: per 32 linear brick indices the occupancy word and its first record

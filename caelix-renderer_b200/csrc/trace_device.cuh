@@ -222,9 +222,11 @@ __device__ __forceinline__ float brick_primitive(const uint32_t* __restrict__ re
 {
     const uint2 info = __ldg(reinterpret_cast<const uint2*>(rec));
     const uint32_t tb = info.y;
-    const float tmin_v[3] = {(float)(tb & 7u), (float)((tb >> 3) & 7u), (float)((tb >> 6) & 7u)};
-    const float tmax_v[3] = {(float)((tb >> 9) & 7u) + 1.0f, (float)((tb >> 12) & 7u) + 1.0f,
-                             (float)((tb >> 15) & 7u) + 1.0f};
+    // Three-bit numbers to floats in the mantissa of 2^23: conversions run at an eighth of the rate (and
+    // kept that pipe at 69 % of its peak here).
+    const auto small = [](uint32_t v) { return __uint_as_float(0x4B000000u | (v & 7u)) - 8388608.0f; };
+    const float tmin_v[3] = {small(tb), small(tb >> 3), small(tb >> 6)};
+    const float tmax_v[3] = {small(tb >> 9) + 1.0f, small(tb >> 12) + 1.0f, small(tb >> 15) + 1.0f};
     float tmin[3], tmax[3], largest, smallest;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -268,10 +270,117 @@ struct Hit
     float object_hit[3];
 };
 
-// Closest hit over the bricks (front-to-back DDA over the brick grid). Cell c of axis k is brick
-// key origin[k] + c, voxels [8 (origin[k] + c), 8 (origin[k] + c + 1)). The next boundary of each
-// axis (nb, exact in fp32: at most 2^24), its distance (tn), the linear cell index and the cells left
-// on the axis are kept and only the stepped axis's are renewed.
+// The walk of a ray over the brick grid, front to back. Cell c of axis k is brick key origin[k] + c,
+// voxels [8 (origin[k] + c), 8 (origin[k] + c + 1)). The next boundary of each axis (nb, exact in fp32:
+// at most 2^24), its distance (tn), the linear cell index and the cells left on the axis are kept and
+// only the stepped axis's are renewed.
+struct RayWalk
+{
+    Ray r;
+    float t_exit, t_max;
+    float nb[3], tn[3];
+    uint32_t left[3];  // cells after this one on the way of the axis
+    uint32_t lin, lin_step[3];
+};
+
+// False: the ray misses the grid.
+__device__ __forceinline__ bool walk_begin(const SceneView& s, const float o[3], const float d[3], float tmin_ray,
+                                           float tmax_ray, RayWalk& w)
+{
+    w.r = make_ray(o, d);
+    float tnear = -3.0e38f, tfar = 3.0e38f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float t0 = (s.low[k] - o[k]) * w.r.inv[k];
+        const float t1 = (s.high[k] - o[k]) * w.r.inv[k];
+        tnear = hmax(tnear, hmin(t0, t1));
+        tfar = hmin(tfar, hmax(t0, t1));
+    }
+    const float t_enter = hmax(tnear, tmin_ray);
+    w.t_exit = hmin(tfar, tmax_ray);
+    w.t_max = tmax_ray;
+    if (!(t_enter <= w.t_exit)) return false;
+    w.lin = 0;
+    uint32_t stride = 1;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float p = o[k] + d[k] * t_enter;
+        int c = (int)floorf(p * 0.125f) - s.origin[k];
+        c = c < 0 ? 0 : c;
+        c = c > (int)s.grid[k] - 1 ? (int)s.grid[k] - 1 : c;
+        const bool up = d[k] >= 0.0f;
+        w.left[k] = up ? s.grid[k] - 1u - (uint32_t)c : (uint32_t)c;
+        w.nb[k] = (float)((s.origin[k] + c + (up ? 1 : 0)) * 8);
+        w.tn[k] = (w.nb[k] - o[k]) * w.r.inv[k];
+        w.lin += (uint32_t)c * stride;
+        w.lin_step[k] = up ? stride : 0u - stride;
+        stride *= s.grid[k];
+    }
+    return true;
+}
+
+// To the next cell on the ray: across the nearest boundary (the first axis of equals). False past the
+// ray's end or the grid's.
+__device__ __forceinline__ bool walk_step(RayWalk& w)
+{
+    int axis = 0;
+    float t_next = w.tn[0];
+    if (w.tn[1] < t_next) {
+        axis = 1;
+        t_next = w.tn[1];
+    }
+    if (w.tn[2] < t_next) {
+        axis = 2;
+        t_next = w.tn[2];
+    }
+    bool out = t_next > w.t_exit;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (axis == k) {
+            out |= w.left[k] == 0u;
+            w.left[k] -= 1u;
+            w.lin += w.lin_step[k];
+            w.nb[k] += w.r.d[k] >= 0.0f ? 8.0f : -8.0f;
+            w.tn[k] = (w.nb[k] - w.r.o[k]) * w.r.inv[k];
+        }
+    }
+    return !out;
+}
+
+// The brick of the walk's cell, record `rec`: true for a hit in [tmin_ray, t_max), at t with `attrib`.
+__device__ __forceinline__ bool walk_brick(const SceneView& s, const RayWalk& w, uint32_t rec, float tmin_ray, float& t,
+                                           uint32_t& attrib)
+{
+    float bo[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) bo[k] = w.nb[k] - (w.r.d[k] >= 0.0f ? 8.0f : 0.0f);
+    t = brick_primitive(s.records + (uint64_t)rec * kRecordWords, w.r, w.t_max, bo, s.enc, attrib);
+    return attrib != 0u && t >= tmin_ray && t < w.t_max;
+}
+
+// The hit found by walk_brick (the walk still at its cell).
+__device__ __forceinline__ Hit walk_hit(const SceneView& s, const RayWalk& w, uint32_t rec, float t, uint32_t attrib)
+{
+    Hit h;
+    h.hit = true;
+    h.t = t;
+    h.attrib = attrib;
+    h.record = rec;
+    const uint32_t gs = s.group_shift;
+    uint32_t cell[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) cell[k] = w.r.d[k] >= 0.0f ? s.grid[k] - 1u - w.left[k] : w.left[k];
+    h.group = (cell[0] >> gs) + s.groups[0] * ((cell[1] >> gs) + s.groups[1] * (cell[2] >> gs));
+    const uint32_t f = (uint32_t)(__ffs(attrib & 0x3Fu) - 1);
+    h.normal[0] = f == 0 ? 1.0f : (f == 1 ? -1.0f : 0.0f);
+    h.normal[1] = f == 2 ? 1.0f : (f == 3 ? -1.0f : 0.0f);
+    h.normal[2] = f == 4 ? 1.0f : (f == 5 ? -1.0f : 0.0f);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) h.object_hit[k] = w.r.o[k] + w.r.d[k] * t;
+    return h;
+}
+
+// Closest hit over the bricks.
 //
 // Issue-bound, on few lanes of a warp (5.4 of 32 before this form: the lanes' brick tests are of
 // unequal length): what counts is instructions per brick and per cell, and how often a warp runs the
@@ -283,93 +392,19 @@ struct Hit
 // voxel steps before lanes outside a brick are served: the same), the walk's state held across it.
 __device__ __forceinline__ Hit trace_ray_body(const SceneView& s, const float o[3], const float d[3], float tmin_ray, float tmax_ray)
 {
-    Hit h;
-    h.hit = false;
-    const Ray r = make_ray(o, d);
-    float tnear = -3.0e38f, tfar = 3.0e38f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float t0 = ((float)(8 * s.origin[k]) - o[k]) * r.inv[k];
-        const float t1 = ((float)(8 * (s.origin[k] + (int)s.grid[k])) - o[k]) * r.inv[k];
-        tnear = hmax(tnear, hmin(t0, t1));
-        tfar = hmin(tfar, hmax(t0, t1));
-    }
-    const float t_enter = hmax(tnear, tmin_ray);
-    const float t_exit = hmin(tfar, tmax_ray);
-    if (!(t_enter <= t_exit)) return h;
-    uint32_t left[3];  // cells after this one on the way of the axis
-    float nb[3], tn[3];
-    uint32_t lin = 0, stride = 1;
-    uint32_t lin_step[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float p = o[k] + d[k] * t_enter;
-        int c = (int)floorf(p * 0.125f) - s.origin[k];
-        c = c < 0 ? 0 : c;
-        c = c > (int)s.grid[k] - 1 ? (int)s.grid[k] - 1 : c;
-        const bool up = d[k] >= 0.0f;
-        left[k] = up ? s.grid[k] - 1u - (uint32_t)c : (uint32_t)c;
-        nb[k] = (float)((s.origin[k] + c + (up ? 1 : 0)) * 8);
-        tn[k] = (nb[k] - o[k]) * r.inv[k];
-        lin += (uint32_t)c * stride;
-        lin_step[k] = up ? stride : 0u - stride;
-        stride *= s.grid[k];
-    }
-    const uint2* __restrict__ cells = s.cells;
-    // To the next cell on the ray: across the nearest boundary (the first axis of equals). False past
-    // the ray's end or the grid's.
-    const auto advance = [&]() {
-        int axis = 0;
-        float t_next = tn[0];
-        if (tn[1] < t_next) {
-            axis = 1;
-            t_next = tn[1];
-        }
-        if (tn[2] < t_next) {
-            axis = 2;
-            t_next = tn[2];
-        }
-        bool out = t_next > t_exit;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            if (axis == k) {
-                out |= left[k] == 0u;
-                left[k] -= 1u;
-                lin += lin_step[k];
-                nb[k] += d[k] >= 0.0f ? 8.0f : -8.0f;
-                tn[k] = (nb[k] - o[k]) * r.inv[k];
-            }
-        }
-        return !out;
-    };
+    Hit miss;
+    miss.hit = false;
+    RayWalk w;
+    if (!walk_begin(s, o, d, tmin_ray, tmax_ray, w)) return miss;
     for (;;) {
-        uint32_t rec;
-        while ((rec = cell_record(cells, lin)) == 0xFFFFFFFFu)
-            if (!advance()) return h;
-        float bo[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) bo[k] = nb[k] - (d[k] >= 0.0f ? 8.0f : 0.0f);
+        uint2 cell;
+        while (!cell_occupied(s.cells, w.lin, cell))
+            if (!walk_step(w)) return miss;
+        const uint32_t rec = cell_record(cell, w.lin);
+        float t;
         uint32_t attrib;
-        const float t = brick_primitive(s.records + (uint64_t)rec * kRecordWords, r, tmax_ray, bo, s.enc, attrib);
-        if (attrib != 0u && t >= tmin_ray && t < tmax_ray) {
-            h.hit = true;
-            h.t = t;
-            h.attrib = attrib;
-            h.record = rec;
-            const uint32_t gs = s.group_shift;
-            uint32_t cell[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) cell[k] = d[k] >= 0.0f ? s.grid[k] - 1u - left[k] : left[k];
-            h.group = (cell[0] >> gs) + s.groups[0] * ((cell[1] >> gs) + s.groups[1] * (cell[2] >> gs));
-            const uint32_t f = (uint32_t)(__ffs(attrib & 0x3Fu) - 1);
-            h.normal[0] = f == 0 ? 1.0f : (f == 1 ? -1.0f : 0.0f);
-            h.normal[1] = f == 2 ? 1.0f : (f == 3 ? -1.0f : 0.0f);
-            h.normal[2] = f == 4 ? 1.0f : (f == 5 ? -1.0f : 0.0f);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) h.object_hit[k] = o[k] + d[k] * t;
-            return h;
-        }
-        if (!advance()) return h;
+        if (walk_brick(s, w, rec, tmin_ray, t, attrib)) return walk_hit(s, w, rec, t, attrib);
+        if (!walk_step(w)) return miss;
     }
 }
 

@@ -29,6 +29,45 @@ def frames(cuda_device, scene, camera):
     return out
 
 
+@pytest.mark.parametrize("paths", [(1 << 17) - 32, (1 << 17) + 32, 3 << 17])
+@pytest.mark.parametrize("origin", [(0, 0, 0), (-37, 1000, -2000)])
+def test_refilled_rays_equal(cuda_device, paths, origin):
+    """Waves on both sides of the 2^17 paths from which finished lanes take new rays: the per-pixel
+    kernel's frame, on a sparse grid far from the origin and on one at it; two views of a batch, whose
+    rays share the warps, equal their plain renders."""
+    import torch
+
+    import caelix_b200
+
+    vs = workloads.noise_world(grid_bricks=(20, 9, 14), brick_occupancy=0.15, emissive_fraction=0.05, seed=21)
+    camera = dict(vs.camera)
+    camera["position"] = camera["position"] + 8.0 * np.asarray(origin, np.float32)
+    vs = vs.like(keys=vs.keys + np.asarray(origin, np.int32))
+    scene = caelix_b200.Scene.from_voxel_scene(cuda_device, vs)
+    r = caelix_b200.Renderer(cuda_device, scene)
+    w, h = paths // 4 // 64, 64 * 4  # whole 8 x 4 blocks, or a block more than whole rows
+    images = []
+    for mode in (r.TRACE_MEGAKERNEL, r.TRACE_WAVEFRONT):
+        r.set_trace_mode(mode, 0)
+        image = torch.full((h, w, 3), -1.0, device="cuda")
+        r.render(image, w, h, camera, bounces=3, seed=9)
+        st = r.stats()
+        images.append((image.cpu().numpy().tobytes(), st.primary_rays, st.bounce_rays, st.shadow_rays))
+    assert images[0] == images[1]
+    outs = [torch.zeros(h * w * 3, device="cuda"), torch.zeros(96 * 96 * 3, device="cuda")]
+    batch = caelix_b200.Batch(cuda_device, [(r, outs[0], w, h, camera, 3, 9, 1), (r, outs[1], 96, 96, camera, 2, 4, 1)])
+    batch.run()
+    torch.cuda.synchronize()
+    assert outs[0].cpu().numpy().tobytes() == images[0][0]
+    ref = torch.zeros_like(outs[1])
+    r.render(ref, 96, 96, camera, bounces=2, seed=4)
+    torch.cuda.synchronize()
+    assert torch.equal(ref, outs[1])
+    batch.close()
+    r.close()
+    scene.close()
+
+
 @pytest.mark.parametrize("lights", [1, 2, 3, 5, 16, 500])
 def test_walks_equal(cuda_device, lights):
     import caelix_b200
