@@ -1,0 +1,32 @@
+// Launches in a chain: a kernel whose CTAs may start when the last CTA of the kernel before it in the
+// stream exits, instead of after that kernel has completed. The kernel calls grid_wait() before it
+// touches anything that an earlier command wrote: the wait ends when the kernel before it is complete
+// and its writes are visible, and that kernel has waited for the one before it. The command before a
+// chained launch must be a kernel; after a copy or a memset the chain starts with a plain launch.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace cx {
+
+__device__ __forceinline__ void grid_wait() { cudaGridDependencySynchronize(); }
+
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), uint32_t grid, uint32_t threads, size_t shared, cudaStream_t stream,
+                           Args... args)
+{
+    cudaLaunchAttribute chained;
+    chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    chained.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = shared;
+    config.stream = stream;
+    config.attrs = &chained;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
+}  // namespace cx

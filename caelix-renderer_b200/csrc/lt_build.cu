@@ -2,6 +2,7 @@
 #include <cuda/atomic>
 
 #include "cx_device.cuh"
+#include "launch.cuh"
 #include "lookback.cuh"
 #include "lt_build.cuh"
 #include "radix_sort.cuh"
@@ -253,6 +254,19 @@ __device__ __forceinline__ void decode_bounds(const BuildControl* control, float
     }
 }
 
+// The Morton code of a box centre (emit: 0.5 (lo + hi)).
+__device__ __forceinline__ uint32_t centre_key(const float4 ctr, const float lo[3], const float extent[3])
+{
+    const float centre[3] = {ctr.x, ctr.y, ctr.z};
+    uint32_t cell[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float q = hmin(hmax((centre[k] - lo[k]) / extent[k] * 1024.0f, 0.0f), 1023.0f);
+        cell[k] = (uint32_t)q;
+    }
+    return morton30(cell[0], cell[1], cell[2]);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Morton codes (value = leaf index) from the box centres the emit wrote + the four digit histograms
 // + clearing the arrival counters and the range-count differences.
@@ -261,6 +275,7 @@ __global__ void __launch_bounds__(kThreads)
                      uint32_t* __restrict__ keys, uint32_t* __restrict__ counter, uint32_t* __restrict__ cover,
                      uint32_t* __restrict__ hist)
 {
+    grid_wait();
     __shared__ uint32_t s_hist[4][kRadix];
     for (int i = threadIdx.x; i < 4 * kRadix; i += blockDim.x) (&s_hist[0][0])[i] = 0;
     float lo[3], hi[3];
@@ -270,15 +285,7 @@ __global__ void __launch_bounds__(kThreads)
     for (int k = 0; k < 3; ++k) extent[k] = hmax(hi[k] - lo[k], 1e-6f);
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 ctr = __ldg(centres + i);  // the world box centre (emit: 0.5 (lo + hi))
-        const float centre[3] = {ctr.x, ctr.y, ctr.z};
-        uint32_t cell[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float q = hmin(hmax((centre[k] - lo[k]) / extent[k] * 1024.0f, 0.0f), 1023.0f);
-            cell[k] = (uint32_t)q;
-        }
-        const uint32_t key = morton30(cell[0], cell[1], cell[2]);
+        const uint32_t key = centre_key(__ldg(centres + i), lo, extent);
         keys[i] = key;
         counter[i] = 0;
         cover[i] = 0;
@@ -296,23 +303,26 @@ __global__ void __launch_bounds__(kThreads)
 // Karras 2012 binary radix tree over the sorted keys; ties broken by sorted position. Also the
 // range-count differences: node i covers the leaf boundaries [a, b) of its range [a, b], so
 // cover[a] += 1, cover[b] -= 1 (their prefix sum counts the nodes over every boundary).
-__device__ __forceinline__ int lt_delta(const uint32_t* __restrict__ keys, int i, int j, int n, uint32_t key_i)
+template <typename KeyAt>
+__device__ __forceinline__ int lt_delta(const KeyAt& key_at, int i, int j, int n, uint32_t key_i)
 {
     if (j < 0 || j >= n) return -1;
-    const uint32_t key_j = __ldg(keys + j);
+    const uint32_t key_j = key_at(j);
     if (key_i == key_j) return 32 + __clz((uint32_t)i ^ (uint32_t)j);
     return __clz(key_i ^ key_j);
 }
 
-__global__ void __launch_bounds__(kThreads)
-    lt_karras_kernel(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ left,
-                     uint32_t* __restrict__ right, uint32_t* __restrict__ parent, uint32_t* __restrict__ leaf_parent,
-                     uint32_t* __restrict__ cover, uint32_t* __restrict__ range_end)
+// Node i: its children and the ends of its leaf range (a <= b, i one of them).
+struct KarrasNode
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    if (i == 0) parent[0] = kNone;
-    const uint32_t key_i = __ldg(keys + i);
+    uint32_t left, right;
+    int a, b;
+};
+
+template <typename KeyAt>
+__device__ __forceinline__ KarrasNode karras_node(const KeyAt& keys, int i, int n)
+{
+    const uint32_t key_i = keys(i);
     const int d = lt_delta(keys, i, i + 1, n, key_i) - lt_delta(keys, i, i - 1, n, key_i) >= 0 ? 1 : -1;
     const int delta_min = lt_delta(keys, i, i - d, n, key_i);
     // The searches with shifts for the divisions by powers of two (lengths are positive, so the
@@ -334,19 +344,178 @@ __global__ void __launch_bounds__(kThreads)
         step2 = (int)(((uint32_t)length + ((1u << shift) - 1u)) >> shift);
     }
     const int gamma = i + split * d + min(d, 0);
-    const int a = min(i, j);
-    const int b = max(i, j);
-    const uint32_t l = a == gamma ? (kChildLeafBit | (uint32_t)gamma) : (uint32_t)gamma;
-    const uint32_t r = b == gamma + 1 ? (kChildLeafBit | (uint32_t)(gamma + 1)) : (uint32_t)(gamma + 1);
-    left[i] = l;
-    right[i] = r;
-    if (l & kChildLeafBit) leaf_parent[l & ~kChildLeafBit] = (uint32_t)i;
-    else parent[l] = (uint32_t)i;
-    if (r & kChildLeafBit) leaf_parent[r & ~kChildLeafBit] = (uint32_t)i;
-    else parent[r] = (uint32_t)i;
-    range_end[i] = (uint32_t)j;
-    atomicAdd(cover + a, 1u);
-    atomicAdd(cover + b, 0xFFFFFFFFu);
+    KarrasNode o;
+    o.a = min(i, j);
+    o.b = max(i, j);
+    o.left = o.a == gamma ? (kChildLeafBit | (uint32_t)gamma) : (uint32_t)gamma;
+    o.right = o.b == gamma + 1 ? (kChildLeafBit | (uint32_t)(gamma + 1)) : (uint32_t)(gamma + 1);
+    return o;
+}
+
+__device__ __forceinline__ void store_node(const KarrasNode& o, uint32_t i, uint32_t* left, uint32_t* right, uint32_t* parent,
+                                           uint32_t* leaf_parent, uint32_t* range_end)
+{
+    if (i == 0) parent[0] = kNone;
+    left[i] = o.left;
+    right[i] = o.right;
+    if (o.left & kChildLeafBit) leaf_parent[o.left & ~kChildLeafBit] = i;
+    else parent[o.left] = i;
+    if (o.right & kChildLeafBit) leaf_parent[o.right & ~kChildLeafBit] = i;
+    else parent[o.right] = i;
+    range_end[i] = (uint32_t)(o.a == (int)i ? o.b : o.a);
+}
+
+__global__ void __launch_bounds__(kThreads)
+    lt_karras_kernel(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ left,
+                     uint32_t* __restrict__ right, uint32_t* __restrict__ parent, uint32_t* __restrict__ leaf_parent,
+                     uint32_t* __restrict__ cover, uint32_t* __restrict__ range_end)
+{
+    grid_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n - 1) return;
+    const KarrasNode o = karras_node([&](int j) { return __ldg(keys + j); }, i, n);
+    store_node(o, (uint32_t)i, left, right, parent, leaf_parent, range_end);
+    atomicAdd(cover + o.a, 1u);
+    atomicAdd(cover + o.b, 0xFFFFFFFFu);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Builds of 2 to kSmallSortKeys leaves, where every kernel is latency, not work. The sort: a warp per
+// leaf places it by its rank (the smaller keys and the equal keys before it: the stable order), counted
+// over a copy of the keys in shared memory. Karras: each CTA searches in a copy of the sorted keys in
+// shared memory. The scans: one CTA. SMALL_MEASURED
+__global__ void __launch_bounds__(kThreads)
+    lt_small_keys_kernel(const float4* __restrict__ centres, uint32_t n, const BuildControl* __restrict__ control,
+                         uint32_t* __restrict__ keys, uint32_t* __restrict__ counter, uint32_t* __restrict__ cover)
+{
+    grid_wait();
+    const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= n) return;
+    float lo[3], hi[3], extent[3];
+    decode_bounds(control, lo, hi);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) extent[k] = hmax(hi[k] - lo[k], 1e-6f);
+    keys[i] = centre_key(__ldg(centres + i), lo, extent);
+    counter[i] = 0;
+    cover[i] = 0;
+}
+
+constexpr uint32_t kRankThreads = 512;
+constexpr uint32_t kRankLeaves = kRankThreads / 32;  // per CTA
+
+// The first n keys into shared memory (the arrays are carved on 256-byte boundaries: whole 16-byte
+// words may be read), the words past them filled with a value above every key.
+template <uint32_t kCta>
+__device__ __forceinline__ void copy_keys(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* s_keys, uint32_t padded)
+{
+#pragma unroll 4
+    for (uint32_t j = threadIdx.x; j < padded / 4; j += kCta) {
+        uint4 v = make_uint4(kNone, kNone, kNone, kNone);
+        if (4 * j < n) v = __ldg(reinterpret_cast<const uint4*>(keys) + j);
+        if (4 * j + 1 >= n) v.y = kNone;
+        if (4 * j + 2 >= n) v.z = kNone;
+        if (4 * j + 3 >= n) v.w = kNone;
+        reinterpret_cast<uint4*>(s_keys)[j] = v;
+    }
+}
+
+__global__ void __launch_bounds__(kRankThreads)
+    lt_rank_sort_kernel(const uint32_t* __restrict__ keys_in, uint32_t n, uint32_t* __restrict__ keys,
+                        uint32_t* __restrict__ values)
+{
+    __shared__ __align__(16) uint32_t s_keys[kSmallSortKeys];
+    grid_wait();
+    const uint32_t padded = (n + 127u) & ~127u;  // whole rows of 32 lanes' 16-byte words
+    copy_keys<kRankThreads>(keys_in, n, s_keys, padded);
+    __syncthreads();
+    const uint32_t i = blockIdx.x * kRankLeaves + threadIdx.x / 32;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (i >= n) return;
+    const uint32_t key = s_keys[i];
+    uint32_t rank = 0;
+#pragma unroll 4
+    for (uint32_t j = lane; j < padded / 4; j += 32) {
+        const uint4 v = reinterpret_cast<const uint4*>(s_keys)[j];
+        const uint32_t below = j < i / 4 ? key + 1u : key;  // equal keys count before element i
+        rank += (v.x < below) + (v.y < below) + (v.z < below) + (v.w < below);
+    }
+    // The equal keys before i in its own word.
+    if (lane < (i & 3u)) rank += s_keys[(i & ~3u) + lane] == key ? 1u : 0u;
+    rank = __reduce_add_sync(0xFFFFFFFFu, rank);
+    if (lane == 0) {
+        keys[rank] = key;
+        values[rank] = i;
+    }
+}
+
+constexpr uint32_t kSmallKarrasThreads = 64;
+
+__global__ void __launch_bounds__(kSmallKarrasThreads)
+    lt_small_karras_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ left,
+                           uint32_t* __restrict__ right, uint32_t* __restrict__ parent, uint32_t* __restrict__ leaf_parent,
+                           uint32_t* __restrict__ cover, uint32_t* __restrict__ range_end)
+{
+    __shared__ __align__(16) uint32_t s_keys[kSmallSortKeys];
+    grid_wait();
+    copy_keys<kSmallKarrasThreads>(keys, n, s_keys, (n + 3u) & ~3u);
+    __syncthreads();
+    const uint32_t i = blockIdx.x * kSmallKarrasThreads + threadIdx.x;
+    if (i + 1 >= n) return;
+    const KarrasNode o = karras_node([&](int j) { return s_keys[j]; }, (int)i, (int)n);
+    store_node(o, i, left, right, parent, leaf_parent, range_end);
+    atomicAdd(cover + o.a, 1u);
+    atomicAdd(cover + o.b, 0xFFFFFFFFu);
+}
+
+constexpr uint32_t kSmallScanThreads = 1024;
+constexpr uint32_t kSmallScanWarps = kSmallScanThreads / 32;
+constexpr int kSmallScanItems = kSmallSortKeys / kSmallScanThreads;
+static_assert(kSmallScanItems == 4, "nodes per thread");
+
+__global__ void __launch_bounds__(kSmallScanThreads)
+    lt_small_scan_kernel(uint32_t nodes, const uint32_t* __restrict__ left, const uint32_t* __restrict__ cover,
+                         uint32_t* __restrict__ depth, uint32_t* __restrict__ wide, BuildControl* __restrict__ control)
+{
+    __shared__ uint32_t s_cover[kSmallSortKeys];
+    __shared__ uint32_t s_scan[kSmallScanWarps];
+    grid_wait();
+    const uint32_t tid = threadIdx.x;
+    // The nodes over every leaf boundary (an inclusive prefix sum), the depths, the 4-wide indices.
+    const uint32_t first = tid * kSmallScanItems;
+    uint32_t v[kSmallScanItems], sum = 0, all;
+#pragma unroll
+    for (int k = 0; k < kSmallScanItems; ++k) {
+        v[k] = first + k < nodes ? cover[first + k] : 0u;
+        sum += v[k];
+    }
+    uint32_t run = block_exclusive_sum<kSmallScanThreads>(sum, s_scan, all);
+#pragma unroll
+    for (int k = 0; k < kSmallScanItems; ++k) {
+        run += v[k];
+        s_cover[first + k] = run;
+    }
+    __syncthreads();
+    bool deep = false;
+    sum = 0;
+#pragma unroll
+    for (int k = 0; k < kSmallScanItems; ++k) {
+        const uint32_t i = first + k;
+        v[k] = i < nodes ? s_cover[__ldg(left + i) & ~kChildLeafBit] - 1u : 1u;
+        deep = deep || (i < nodes && v[k] >= 128u);
+        sum += (v[k] & 1u) == 0 ? 1u : 0u;
+    }
+    if (deep) atomicOr(&control->status, kStatusDepthGuard);
+    run = block_exclusive_sum<kSmallScanThreads>(sum, s_scan, all);
+    if (tid == 0) control->node_count = all;
+#pragma unroll
+    for (int k = 0; k < kSmallScanItems; ++k) {
+        const uint32_t i = first + k;
+        if (i < nodes) {
+            depth[i] = v[k];
+            wide[i] = run;
+        }
+        run += (v[k] & 1u) == 0 ? 1u : 0u;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -431,6 +600,7 @@ __global__ void __launch_bounds__(kAggTile)
                    uint32_t* __restrict__ crossing, LightBvhLeaf* __restrict__ leaves,
                    LightBvhNode* __restrict__ nodes, BuildControl* control)
 {
+    grid_wait();
     // The arrival counters and the tile's lists are dead once the rows are built: they share
     // their memory with the row staging.
     union Scratch
@@ -627,14 +797,13 @@ __global__ void __launch_bounds__(kAggTile)
 // The walks up through the nodes whose range crosses a tile, from the children the tiles listed
 // (an in-tile node, its summary in its slot, or a leaf): the second thread to arrive at a node
 // computes it and goes on. The walks were run inside the tile kernel at first: chains of
-// dependent device-scope atomics and L2 loads that kept each tile's CTA resident for them. Up to
-// kUpperOneCtaItems walks (one per thread: builds of up to about 16 k leaves) run in one CTA
-// (kOneCta), whose arrivals are block-scope and whose siblings' summaries come through L1; more
-// run on a persistent grid with device-scope arrivals (the list's length is known on the device
-// only: each variant checks it). With six walks per thread (97 k leaves) the one CTA was slower
-// than the grid (the light-tree flush of the 2 M-brick world 0.22 against 0.18 ms).
-constexpr uint32_t kUpperOneCtaItems = 1024;
-constexpr uint32_t kUpperOneCtaThreads = 1024;
+// dependent device-scope atomics and L2 loads that kept each tile's CTA resident for them. Builds of
+// up to kTailLeaves leaves run them in one CTA (kOneCta), whose arrivals are block-scope and whose
+// siblings' summaries come through L1; larger ones on a persistent grid with device-scope arrivals.
+// With six walks per thread (97 k leaves) the one CTA was slower than the grid (the light-tree flush of
+// the 2 M-brick world 0.22 against 0.18 ms).
+constexpr uint32_t kTailLeaves = 16384;
+constexpr uint32_t kTailThreads = 1024;
 
 // A summary written earlier by this kernel's CTA (after an acquire: weak loads through L1).
 __device__ __forceinline__ LightSummary load_summary_weak(const LightSummary* p)
@@ -648,45 +817,115 @@ __device__ __forceinline__ LightSummary load_summary_weak(const LightSummary* p)
     return s;
 }
 
+// The walk from listed child `from`.
 template <bool kOneCta>
-__global__ void __launch_bounds__(kOneCta ? kUpperOneCtaThreads : kThreads)
+__device__ __forceinline__ void upper_walk(uint32_t from, const LightSummary* __restrict__ sorted,
+                                           const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
+                                           const uint32_t* __restrict__ parent, const uint32_t* __restrict__ leaf_parent,
+                                           uint32_t* counter, AggregateSlot* aggregates, BuildControl* control)
+{
+    constexpr cuda::thread_scope kScope = kOneCta ? cuda::thread_scope_block : cuda::thread_scope_device;
+    const bool leaf = (from & kChildLeafBit) != 0;
+    LightSummary cur = leaf ? load_summary_cg(sorted + (from & ~kChildLeafBit)) : load_summary_cg(&aggregates[from].summary);
+    uint32_t node = leaf ? __ldg(leaf_parent + (from & ~kChildLeafBit)) : __ldg(parent + from);
+    uint32_t depth = 0;
+    for (; depth < 128 && node != kNone; ++depth) {
+        const uint32_t l = __ldg(left + node);
+        const uint32_t r = __ldg(right + node);
+        const uint32_t up = __ldg(parent + node);
+        const uint32_t sibling = l == from ? r : l;
+        cuda::atomic_ref<uint32_t, kScope> arrival(counter[node]);
+        if (arrival.fetch_add(1u, cuda::memory_order_acq_rel) == 0) break;
+        LightSummary sib;
+        if (sibling & kChildLeafBit) sib = load_summary_cg(sorted + (sibling & ~kChildLeafBit));
+        else if (kOneCta) sib = load_summary_weak(&aggregates[sibling].summary);
+        else sib = load_summary_cg(&aggregates[sibling].summary);
+        cur = l == from ? lt_union(cur, sib) : lt_union(sib, cur);
+        store_slot(aggregates + node, cur);
+        from = node;
+        node = up;
+    }
+    if (depth == 128) atomicOr(&control->status, kStatusDepthGuard);
+}
+
+__global__ void __launch_bounds__(kThreads)
     lt_aggregate_upper_kernel(const LightSummary* __restrict__ sorted, const uint32_t* __restrict__ left,
                               const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent,
                               const uint32_t* __restrict__ leaf_parent, uint32_t* counter,
                               AggregateSlot* aggregates, const uint32_t* __restrict__ upper, BuildControl* control)
 {
-    constexpr cuda::thread_scope kScope = kOneCta ? cuda::thread_scope_block : cuda::thread_scope_device;
+    grid_wait();
     const uint32_t count = control->upper_count;
-    if (kOneCta ? count > kUpperOneCtaItems : count <= kUpperOneCtaItems) return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        uint32_t from = upper[i];
-        const bool leaf = (from & kChildLeafBit) != 0;
-        LightSummary cur = leaf ? load_summary_cg(sorted + (from & ~kChildLeafBit)) : load_summary_cg(&aggregates[from].summary);
-        uint32_t node = leaf ? __ldg(leaf_parent + (from & ~kChildLeafBit)) : __ldg(parent + from);
-        uint32_t depth = 0;
-        for (; depth < 128 && node != kNone; ++depth) {
-            const uint32_t l = __ldg(left + node);
-            const uint32_t r = __ldg(right + node);
-            const uint32_t up = __ldg(parent + node);
-            const uint32_t sibling = l == from ? r : l;
-            cuda::atomic_ref<uint32_t, kScope> arrival(counter[node]);
-            if (arrival.fetch_add(1u, cuda::memory_order_acq_rel) == 0) break;
-            LightSummary sib;
-            if (sibling & kChildLeafBit) sib = load_summary_cg(sorted + (sibling & ~kChildLeafBit));
-            else if (kOneCta) sib = load_summary_weak(&aggregates[sibling].summary);
-            else sib = load_summary_cg(&aggregates[sibling].summary);
-            cur = l == from ? lt_union(cur, sib) : lt_union(sib, cur);
-            store_slot(aggregates + node, cur);
-            from = node;
-            node = up;
-        }
-        if (depth == 128) atomicOr(&control->status, kStatusDepthGuard);
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+        upper_walk<false>(upper[i], sorted, left, right, parent, leaf_parent, counter, aggregates, control);
 }
 
-// The 4-wide nodes over the even-depth binary nodes that cross a tile (listed by the tile kernel):
-// one thread per node, children and summaries read from the global arrays and slots, the row
-// written by the thread; the parent words of its leaf slots written into the leaves.
+// The 4-wide node over even-depth binary node i, which crosses a tile: children and summaries read
+// from the global arrays and slots, the row written by the thread; the parent words of its leaf slots
+// written into the leaves. count: the 4-wide nodes there is room for.
+template <bool kOneCta>
+__device__ __forceinline__ void upper_row(uint32_t i, uint32_t n, uint32_t count, const uint32_t* __restrict__ values,
+                                          const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
+                                          const uint32_t* __restrict__ parent, const uint32_t* __restrict__ wide,
+                                          const LightSummary* __restrict__ sorted, const AggregateSlot* aggregates,
+                                          LightBvhLeaf* __restrict__ leaves, LightBvhNode* __restrict__ nodes)
+{
+    const uint32_t w = __ldg(wide + i);
+    if (w >= count) return;
+    uint32_t slots[4];
+    wide_slots(__ldg(left + i), __ldg(right + i),
+               [&](uint32_t x) { return make_uint2(__ldg(left + x), __ldg(right + x)); }, slots);
+    uint4* row = reinterpret_cast<uint4*>(nodes + w);
+    LightSummary sm[4];
+    uint32_t word[4];
+#pragma unroll
+    for (uint32_t c = 0; c < 4; ++c) {
+#pragma unroll
+        for (int f = 0; f < 6; ++f) sm[c].face[f] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sm[c].lo[k] = sm[c].hi[k] = 0.0f;
+        word[c] = kNone;
+        const uint32_t slot = slots[c];
+        if (slot == kNone) continue;
+        if (slot & kChildLeafBit) {
+            const uint32_t p = slot & ~kChildLeafBit;
+            sm[c] = load_summary_cg(sorted + p);
+            const uint32_t leaf = __ldg(values + p);
+            word[c] = kChildLeafBit | leaf;
+            leaves[leaf].parent = (w << kParentSlotBits) | c;  // the leaf's parent word, in place
+        } else {
+            sm[c] = kOneCta ? load_summary_weak(&aggregates[slot].summary) : load_summary_cg(&aggregates[slot].summary);
+            word[c] = __ldg(wide + slot);
+        }
+    }
+    float f[48];
+#pragma unroll
+    for (uint32_t wd = 0; wd < 48; ++wd) {
+        uint32_t c, idx;
+        row_word(wd, c, idx);
+        f[wd] = reinterpret_cast<const float*>(&sm[c])[idx];
+    }
+#pragma unroll
+    for (int u = 0; u < 12; ++u) row[u] = make_uint4(__float_as_uint(f[4 * u]), __float_as_uint(f[4 * u + 1]),
+                                                     __float_as_uint(f[4 * u + 2]), __float_as_uint(f[4 * u + 3]));
+    row[12] = make_uint4(word[0], word[1], word[2], word[3]);
+    // The node's own parent link.
+    uint32_t up_node = kNone, up_slot = 0;
+    if (i != 0) {
+        const uint32_t p = __ldg(parent + i);
+        const uint32_t g = p + 1 < n ? __ldg(parent + p) : kNone;
+        if (g + 1 < n) {
+            const uint32_t gl = __ldg(left + g);
+            const uint32_t b0 = p == gl ? 0u : ((gl & kChildLeafBit) ? 1u : 2u);
+            up_slot = b0 + (__ldg(right + p) == i ? 1u : 0u);
+            up_node = __ldg(wide + g);
+        }
+    }
+    row[13] = make_uint4(up_node, up_slot, 0u, 0u);
+}
+
+// The 4-wide nodes over the even-depth nodes that cross a tile (listed by the tile kernel): one thread
+// per node.
 __global__ void __launch_bounds__(kThreads)
     lt_wide_upper_kernel(uint32_t n, uint32_t node_capacity, const uint32_t* __restrict__ values,
                          const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
@@ -695,63 +934,11 @@ __global__ void __launch_bounds__(kThreads)
                          const AggregateSlot* __restrict__ aggregates, LightBvhLeaf* __restrict__ leaves,
                          LightBvhNode* __restrict__ nodes, const BuildControl* __restrict__ control)
 {
+    grid_wait();
     const uint32_t count = min(control->node_count, node_capacity);
     const uint32_t listed = control->crossing_count;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < listed; t += gridDim.x * blockDim.x) {
-        const uint32_t i = crossing[t];
-        const uint32_t w = __ldg(wide + i);
-        if (w >= count) continue;
-        uint32_t slots[4];
-        wide_slots(__ldg(left + i), __ldg(right + i),
-                   [&](uint32_t x) { return make_uint2(__ldg(left + x), __ldg(right + x)); }, slots);
-        uint4* row = reinterpret_cast<uint4*>(nodes + w);
-        LightSummary sm[4];
-        uint32_t word[4];
-#pragma unroll
-        for (uint32_t c = 0; c < 4; ++c) {
-#pragma unroll
-            for (int f = 0; f < 6; ++f) sm[c].face[f] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) sm[c].lo[k] = sm[c].hi[k] = 0.0f;
-            word[c] = kNone;
-            const uint32_t slot = slots[c];
-            if (slot == kNone) continue;
-            if (slot & kChildLeafBit) {
-                const uint32_t p = slot & ~kChildLeafBit;
-                sm[c] = load_summary_cg(sorted + p);
-                const uint32_t leaf = __ldg(values + p);
-                word[c] = kChildLeafBit | leaf;
-                leaves[leaf].parent = (w << kParentSlotBits) | c;  // the leaf's parent word, in place
-            } else {
-                sm[c] = load_summary_cg(&aggregates[slot].summary);
-                word[c] = __ldg(wide + slot);
-            }
-        }
-        float f[48];
-#pragma unroll
-        for (uint32_t wd = 0; wd < 48; ++wd) {
-            uint32_t c, idx;
-            row_word(wd, c, idx);
-            f[wd] = reinterpret_cast<const float*>(&sm[c])[idx];
-        }
-#pragma unroll
-        for (int u = 0; u < 12; ++u) row[u] = make_uint4(__float_as_uint(f[4 * u]), __float_as_uint(f[4 * u + 1]),
-                                                         __float_as_uint(f[4 * u + 2]), __float_as_uint(f[4 * u + 3]));
-        row[12] = make_uint4(word[0], word[1], word[2], word[3]);
-        // The node's own parent link.
-        uint32_t up_node = kNone, up_slot = 0;
-        if (i != 0) {
-            const uint32_t p = __ldg(parent + i);
-            const uint32_t g = p + 1 < n ? __ldg(parent + p) : kNone;
-            if (g + 1 < n) {
-                const uint32_t gl = __ldg(left + g);
-                const uint32_t b0 = p == gl ? 0u : ((gl & kChildLeafBit) ? 1u : 2u);
-                up_slot = b0 + (__ldg(right + p) == i ? 1u : 0u);
-                up_node = __ldg(wide + g);
-            }
-        }
-        row[13] = make_uint4(up_node, up_slot, 0u, 0u);
-    }
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < listed; t += gridDim.x * blockDim.x)
+        upper_row<false>(crossing[t], n, count, values, left, right, parent, wide, sorted, aggregates, leaves, nodes);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -799,6 +986,7 @@ __global__ void __launch_bounds__(kScanThreads)
     lt_cover_scan_kernel(uint32_t count, uint32_t* cover, uint32_t* states, uint32_t* tile_counter,
                          BuildControl* control)
 {
+    grid_wait();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_scan[kScanThreads / 32];
     __shared__ uint32_t s_prefix;
@@ -837,6 +1025,7 @@ __global__ void __launch_bounds__(kScanThreads)
                          uint32_t* __restrict__ depth_out, uint32_t* __restrict__ wide, uint32_t* states,
                          uint32_t* tile_counter, BuildControl* control)
 {
+    grid_wait();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_scan[kScanThreads / 32];
     __shared__ uint32_t s_prefix;
@@ -880,9 +1069,9 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // ---------------------------------------------------------------------------------------------
 // The header (one thread): root summary, counts, overflow; the one-leaf tree's single node.
-__global__ void lt_finish_kernel(uint32_t n, uint32_t found, uint32_t node_capacity, LightBvhLeaf* leaves,
-                                 LightBvhNode* nodes, const AggregateSlot* aggregates, LightTreeHeader* header,
-                                 LightTreeState* state, const BuildControl* control)
+__device__ __forceinline__ void finish_build(uint32_t n, uint32_t found, uint32_t node_capacity, LightBvhLeaf* leaves,
+                                             LightBvhNode* nodes, const AggregateSlot* aggregates, LightTreeHeader* header,
+                                             LightTreeState* state, const BuildControl* control)
 {
     LightSummary root;
 #pragma unroll
@@ -928,6 +1117,36 @@ __global__ void lt_finish_kernel(uint32_t n, uint32_t found, uint32_t node_capac
         state->bounds[k] = lo[k];
         state->bounds[3 + k] = hi[k];
     }
+}
+
+__global__ void lt_finish_kernel(uint32_t n, uint32_t found, uint32_t node_capacity, LightBvhLeaf* leaves,
+                                 LightBvhNode* nodes, const AggregateSlot* aggregates, LightTreeHeader* header,
+                                 LightTreeState* state, const BuildControl* control)
+{
+    grid_wait();
+    finish_build(n, found, node_capacity, leaves, nodes, aggregates, header, state, control);
+}
+
+// After the tile kernel of a build of 2 to kTailLeaves leaves, by one CTA: the upper walks, the rows over
+// the nodes that cross tiles, the header. TAIL_MEASURED
+__global__ void __launch_bounds__(kTailThreads)
+    lt_tail_kernel(uint32_t n, uint32_t found, uint32_t node_capacity, const uint32_t* __restrict__ values,
+                   const LightSummary* __restrict__ sorted, const uint32_t* __restrict__ left,
+                   const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent,
+                   const uint32_t* __restrict__ leaf_parent, const uint32_t* __restrict__ wide, uint32_t* counter,
+                   AggregateSlot* aggregates, const uint32_t* __restrict__ upper, const uint32_t* __restrict__ crossing,
+                   LightBvhLeaf* __restrict__ leaves, LightBvhNode* __restrict__ nodes, LightTreeHeader* header,
+                   LightTreeState* state, BuildControl* control)
+{
+    grid_wait();
+    const uint32_t walks = control->upper_count, rows = control->crossing_count;
+    for (uint32_t i = threadIdx.x; i < walks; i += kTailThreads)
+        upper_walk<true>(upper[i], sorted, left, right, parent, leaf_parent, counter, aggregates, control);
+    __syncthreads();
+    const uint32_t count = min(control->node_count, node_capacity);
+    for (uint32_t i = threadIdx.x; i < rows; i += kTailThreads)
+        upper_row<true>(crossing[i], n, count, values, left, right, parent, wide, sorted, aggregates, leaves, nodes);
+    if (threadIdx.x == 0) finish_build(n, found, node_capacity, leaves, nodes, aggregates, header, state, control);
 }
 
 uint32_t grid_for(uint32_t n, uint32_t per_block, uint32_t cap)
@@ -1037,14 +1256,28 @@ cudaError_t lt_build(const LightBvhBuffers& b, const LightBvhInput& in, cudaStre
             in.records, n, in.record_group, in.record_entry, in.group_frames, in.group_count, b.leaves,
             reinterpret_cast<float4*>(b.aggregates), b.control);  // the slots hold the centres until aggregation
         mark(1);
-        lt_morton_kernel<<<grid_for(n, kThreads * 4, sms * morton_per_sm), kThreads, 0, stream>>>(
-            reinterpret_cast<const float4*>(b.aggregates), n, b.control, b.keys, b.counter, b.cover, b.sort_scratch);
-        mark(2);
-        // The sort (one small-sort CTA up to kSmallSortKeys pairs); later kernels read a sorted
-        // leaf's summary through the permutation.
-        onesweep_sort(b.keys, b.values, b.keys_alt, b.values_alt, n, true, b.sort_scratch, &b.control->status,
-                      stream, nullptr, kpt);
-        mark(3);
+        e = cudaGetLastError();
+        if (n >= 2 && n <= kSmallSortKeys) {
+            if (e == cudaSuccess)
+                e = launch_chained(lt_small_keys_kernel, grid_for(n, kThreads, 1u << 30), kThreads, 0, stream,
+                                   reinterpret_cast<const float4*>(b.aggregates), n, b.control, b.keys_alt, b.counter,
+                                   b.cover);
+            mark(2);
+            if (e == cudaSuccess)
+                e = launch_chained(lt_rank_sort_kernel, (n + kRankLeaves - 1) / kRankLeaves, kRankThreads, 0, stream,
+                                   b.keys_alt, n, b.keys, b.values);
+            mark(3);
+        } else {
+            if (e == cudaSuccess)
+                e = launch_chained(lt_morton_kernel, grid_for(n, kThreads * 4, sms * morton_per_sm), kThreads, 0, stream,
+                                   reinterpret_cast<const float4*>(b.aggregates), n, b.control, b.keys, b.counter, b.cover,
+                                   b.sort_scratch);
+            mark(2);
+            // The sort; later kernels read a sorted leaf's summary through the permutation.
+            onesweep_sort(b.keys, b.values, b.keys_alt, b.values_alt, n, true, b.sort_scratch, &b.control->status, stream,
+                          nullptr, kpt);
+            mark(3);
+        }
     } else {
         mark(1);
         mark(2);
@@ -1053,47 +1286,75 @@ cudaError_t lt_build(const LightBvhBuffers& b, const LightBvhInput& in, cudaStre
     if (n >= 2) {
         const uint32_t nodes = n - 1;
         // values_alt (free after the sort) holds each node's range end.
-        lt_karras_kernel<<<grid_for(nodes, kThreads, 1u << 30), kThreads, 0, stream>>>(
-            b.keys, (int)n, b.left, b.right, b.parent, b.leaf_parent, b.cover, b.values_alt);
-        mark(4);
-        const uint32_t tiles = (nodes + kScanTile - 1) / kScanTile;
-        lt_cover_scan_kernel<<<tiles, kScanThreads, 0, stream>>>(nodes, b.cover, cover_states, scan_counters,
-                                                                  b.control);
-        lt_flags_scan_kernel<<<tiles, kScanThreads, 0, stream>>>(nodes, b.left, b.cover, b.depth, b.wide, flag_states,
-                                                                  scan_counters + 1, b.control);
+        if (n <= kSmallSortKeys) {
+            if (e == cudaSuccess)
+                e = launch_chained(lt_small_karras_kernel, grid_for(nodes, kSmallKarrasThreads, 1u << 30), kSmallKarrasThreads,
+                                   0, stream, b.keys, n, b.left, b.right, b.parent, b.leaf_parent, b.cover, b.values_alt);
+            mark(4);
+            if (e == cudaSuccess)
+                e = launch_chained(lt_small_scan_kernel, 1, kSmallScanThreads, 0, stream, nodes, b.left, b.cover, b.depth,
+                                   b.wide, b.control);
+        } else {
+            if (e == cudaSuccess)
+                e = launch_chained(lt_karras_kernel, grid_for(nodes, kThreads, 1u << 30), kThreads, 0, stream, b.keys, (int)n,
+                                   b.left, b.right, b.parent, b.leaf_parent, b.cover, b.values_alt);
+            mark(4);
+            const uint32_t tiles = (nodes + kScanTile - 1) / kScanTile;
+            if (e == cudaSuccess)
+                e = launch_chained(lt_cover_scan_kernel, tiles, kScanThreads, 0, stream, nodes, b.cover, cover_states,
+                                   scan_counters, b.control);
+            if (e == cudaSuccess)
+                e = launch_chained(lt_flags_scan_kernel, tiles, kScanThreads, 0, stream, nodes, b.left, b.cover, b.depth,
+                                   b.wide, flag_states, scan_counters + 1, b.control);
+        }
         mark(5);
         // cover (free after the flags scan) lists the upper walks, keys_alt (free after the sort) the
         // even-depth nodes that cross a tile.
-        lt_tile_kernel<<<(n + kAggTile - 1) / kAggTile, kAggTile, 0, stream>>>(
-            n, b.node_capacity, b.sorted, b.left, b.right, b.parent, b.leaf_parent, b.values_alt, b.depth, b.wide,
-            b.values, b.aggregates, b.cover, b.keys_alt, b.leaves, b.nodes, b.control);
-        lt_aggregate_upper_kernel<true><<<1, kUpperOneCtaThreads, 0, stream>>>(
-            b.sorted, b.left, b.right, b.parent, b.leaf_parent, b.counter, b.aggregates, b.cover, b.control);
-        lt_aggregate_upper_kernel<false><<<grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream>>>(
-            b.sorted, b.left, b.right, b.parent, b.leaf_parent, b.counter, b.aggregates, b.cover, b.control);
+        if (e == cudaSuccess)
+            e = launch_chained(lt_tile_kernel, (n + kAggTile - 1) / kAggTile, kAggTile, 0, stream, n, b.node_capacity,
+                               b.sorted, b.left, b.right, b.parent, b.leaf_parent, b.values_alt, b.depth, b.wide, b.values,
+                               b.aggregates, b.cover, b.keys_alt, b.leaves, b.nodes, b.control);
+        if (n <= kTailLeaves) {
+            mark(6);
+            if (e == cudaSuccess)
+                e = launch_chained(lt_tail_kernel, 1, kTailThreads, 0, stream, n, found, b.node_capacity, b.values, b.sorted,
+                                   b.left, b.right, b.parent, b.leaf_parent, b.wide, b.counter, b.aggregates, b.cover,
+                                   b.keys_alt, b.leaves, b.nodes, b.header, b.state, b.control);
+            mark(7);
+            return e != cudaSuccess ? e : cudaGetLastError();
+        }
+        if (e == cudaSuccess)
+            e = launch_chained(lt_aggregate_upper_kernel, grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream, b.sorted,
+                               b.left, b.right, b.parent, b.leaf_parent, b.counter, b.aggregates, b.cover, b.control);
         mark(6);
-        lt_wide_upper_kernel<<<grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream>>>(
-            n, b.node_capacity, b.values, b.left, b.right, b.parent, b.keys_alt, b.wide, b.sorted, b.aggregates,
-            b.leaves, b.nodes, b.control);
+        if (e == cudaSuccess)
+            e = launch_chained(lt_wide_upper_kernel, grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream, n,
+                               b.node_capacity, b.values, b.left, b.right, b.parent, b.keys_alt, b.wide, b.sorted,
+                               b.aggregates, b.leaves, b.nodes, b.control);
     } else {
         mark(4);
         mark(5);
         mark(6);
     }
-    lt_finish_kernel<<<1, 1, 0, stream>>>(n, found, b.node_capacity, b.leaves, b.nodes, b.aggregates, b.header,
-                                          b.state, b.control);
+    // (Without leaves the command before is the memset.)
+    if (e == cudaSuccess && n > 0)
+        e = launch_chained(lt_finish_kernel, 1, 1, 0, stream, n, found, b.node_capacity, b.leaves, b.nodes, b.aggregates,
+                           b.header, b.state, b.control);
+    else if (e == cudaSuccess)
+        lt_finish_kernel<<<1, 1, 0, stream>>>(n, found, b.node_capacity, b.leaves, b.nodes, b.aggregates, b.header, b.state,
+                                              b.control);
     mark(7);
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 uint32_t lt_kernel_launches(uint32_t n)
 {
-    // emit, Morton, the sort (one small-sort CTA, or four passes), the seven tree kernels from two
-    // leaves (the upper aggregation's two variants both launch; one of them returns at once),
-    // finish.
-    if (n == 0) return 1;
-    const uint32_t sort = n <= kSmallSortKeys ? 1u : 4u;
-    return 2 + sort + (n >= 2 ? 7u : 0u) + 1;
+    // finish; emit, Morton, sort, finish; emit, keys, sort, Karras, scan, tile,
+    // tail; emit, Morton, four sort passes, Karras, two
+    // scans, tile, then the tail, or upper aggregation, upper rows and finish.
+    if (n <= 1) return n == 0 ? 1u : 4u;
+    if (n <= kSmallSortKeys) return 7;
+    return 10u + (n <= kTailLeaves ? 1u : 3u);
 }
 
 }  // namespace cx

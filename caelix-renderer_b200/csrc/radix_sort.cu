@@ -3,6 +3,7 @@
 #include <atomic>
 
 #include "cx_device.cuh"
+#include "launch.cuh"
 #include "radix_sort.cuh"
 
 namespace cx {
@@ -154,6 +155,7 @@ __device__ __forceinline__ uint32_t digit_lookback(const SortPass& a, uint32_t t
 template <int KPT>
 __global__ void __launch_bounds__(kSortThreads, 4) onesweep_pass_kernel(const SortPass a)
 {
+    grid_wait();
     constexpr int kTile = kSortThreads * KPT;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp_counts[kSortWarps][kRadix];  // counts, then exclusive offsets per warp
@@ -325,6 +327,7 @@ __device__ __forceinline__ void pipe_issue(const SortPass& a, PipeShared& S, uin
 
 __global__ void __launch_bounds__(kSortThreads, 2) onesweep_pipe_kernel(const SortPass a, uint32_t tiles)
 {
+    grid_wait();
     extern __shared__ __align__(128) unsigned char pipe_smem[];
     PipeShared& S = *reinterpret_cast<PipeShared*>(pipe_smem);
     constexpr int KPT = kSortKeysPerThread;
@@ -456,6 +459,7 @@ __global__ void __launch_bounds__(kSortThreads) small_sort_kernel(uint32_t* __re
                                                                   uint32_t* __restrict__ values, uint32_t n,
                                                                   uint32_t passes, const SortGather gather)
 {
+    grid_wait();
     constexpr int KPT = kSmallSortKeysPerThread;
     __shared__ uint32_t s_warp_counts[kSortWarps][kRadix];
     __shared__ uint32_t s_local[kRadix];
@@ -533,6 +537,7 @@ __global__ void __launch_bounds__(kSortThreads) rank_sort_kernel(uint32_t* __res
                                                                  uint32_t* __restrict__ values, uint32_t n,
                                                                  const SortGather gather)
 {
+    grid_wait();
     __shared__ uint32_t s_keys[kRankSortKeys];
     __shared__ uint32_t s_values[kRankSortKeys];
     const uint32_t tid = threadIdx.x;
@@ -580,12 +585,11 @@ void onesweep_sort(uint32_t* keys_a, uint32_t* values_a, uint32_t* keys_b, uint3
     if (n <= kSmallSortKeys) {
         const SortGather g = gather ? *gather : SortGather{nullptr, 0, nullptr, nullptr};
         if (n <= kRankSortKeys) {
-            if (identity_values) rank_sort_kernel<true><<<1, kSortThreads, 0, stream>>>(keys_a, values_a, n, g);
-            else rank_sort_kernel<false><<<1, kSortThreads, 0, stream>>>(keys_a, values_a, n, g);
-        } else if (identity_values) {
-            small_sort_kernel<true><<<1, kSortThreads, 0, stream>>>(keys_a, values_a, n, passes, g);
+            launch_chained(identity_values ? rank_sort_kernel<true> : rank_sort_kernel<false>, 1, kSortThreads, 0, stream, keys_a,
+                           values_a, n, g);
         } else {
-            small_sort_kernel<false><<<1, kSortThreads, 0, stream>>>(keys_a, values_a, n, passes, g);
+            launch_chained(identity_values ? small_sort_kernel<true> : small_sort_kernel<false>, 1, kSortThreads, 0, stream,
+                           keys_a, values_a, n, passes, g);
         }
         return;
     }
@@ -634,10 +638,13 @@ void onesweep_sort(uint32_t* keys_a, uint32_t* values_a, uint32_t* keys_b, uint3
         p.inverse = (last && gather) ? gather->inverse : nullptr;
         p.silent_tile = (pass == 0 && wait_test) ? wait_test->silent_tile : 0xFFFFFFFFu;
         p.spin_limit = wait_test ? wait_test->spin_limit : kSpinLimit;
-        if (pipe) onesweep_pipe_kernel<<<pipe_grid, kSortThreads, sizeof(PipeShared), stream>>>(p, tiles);
-        else if (keys_per_thread == 4) onesweep_pass_kernel<4><<<tiles, kSortThreads, 0, stream>>>(p);
-        else if (keys_per_thread == 8) onesweep_pass_kernel<8><<<tiles, kSortThreads, 0, stream>>>(p);
-        else onesweep_pass_kernel<16><<<tiles, kSortThreads, 0, stream>>>(p);
+        if (pipe)
+            launch_chained(onesweep_pipe_kernel, pipe_grid, kSortThreads, sizeof(PipeShared), stream, p, tiles);
+        else
+            launch_chained(keys_per_thread == 4   ? onesweep_pass_kernel<4>
+                           : keys_per_thread == 8 ? onesweep_pass_kernel<8>
+                                                  : onesweep_pass_kernel<16>,
+                           tiles, kSortThreads, 0, stream, p);
         uint32_t* t = kin;
         kin = kout;
         kout = t;

@@ -20,6 +20,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "launch.cuh"
 #include "trace.cuh"
 #include "trace_device.cuh"
 
@@ -61,10 +62,6 @@ struct WaveGen
     uint32_t count;
     uint32_t block_width;
 };
-
-// Every kernel of a stage starts with this: it may have been launched while the one before it ended
-// (launch), and waits here until that one is complete and its writes are visible.
-__device__ __forceinline__ void wave_begin() { cudaGridDependencySynchronize(); }
 
 // Warp-aggregated append: returns this lane's first index in the queue. All lanes of the warp call.
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, uint32_t n)
@@ -148,7 +145,7 @@ __global__ void __launch_bounds__(kWaveThreads)
 __global__ void __launch_bounds__(kWaveThreads)
     wave_resolve_kernel(const WaveView* __restrict__ views, const WaveGen g, const WaveBuffers b)
 {
-    wave_begin();
+    grid_wait();
     const uint32_t n_views = g.entries / g.samples;
     const uint32_t item = blockIdx.x * kWaveThreads + threadIdx.x;
     const uint32_t per_sample = g.count / g.samples;
@@ -237,7 +234,7 @@ template <bool kEntities>
 __global__ void __launch_bounds__(kWaveThreads)
     wave_trace_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity)
 {
-    wave_begin();
+    grid_wait();
     const uint32_t n = *(volatile uint32_t*)&b.counts[2 * parity];
     begin_stage(b, parity);
     const uint32_t lane = threadIdx.x & 31u;
@@ -275,7 +272,7 @@ constexpr uint32_t kRefillPaths = 1u << 17;  // waves of more paths than this ar
 __global__ void __launch_bounds__(kWaveThreads, 6)
     wave_trace_refill_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity)
 {
-    wave_begin();
+    grid_wait();
     const uint32_t n = *(volatile uint32_t*)&b.counts[2 * parity];
     begin_stage(b, parity);
     uint32_t* const fetch = &b.counts[kFetchTrace + parity];
@@ -462,7 +459,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     wave_shade_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj,
                       bool resolve)
 {
-    wave_begin();
+    grid_wait();
     __shared__ float s_albedo[kMode == kShadeReplay ? kAlbedoCache * 3 : 1];
     __shared__ uint32_t s_tag[kMode == kShadeReplay ? kAlbedoCache : 1];
     AlbedoCache cache{s_tag, s_albedo, adj.d_albedo};
@@ -710,7 +707,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     wave_light_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj,
                       bool resolve)
 {
-    wave_begin();
+    grid_wait();
     __shared__ float s_albedo[kMode == kShadeReplay ? kAlbedoCache * 3 : 1];
     __shared__ uint32_t s_tag[kMode == kShadeReplay ? kAlbedoCache : 1];
     AlbedoCache cache{s_tag, s_albedo, adj.d_albedo};
@@ -1007,23 +1004,13 @@ WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_wi
 
 namespace {
 
-// A launch whose CTAs may start when the last CTA of the launch before it exits (wave_begin waits for
-// that launch's writes), instead of after it has completed. Measured (one B200): 160 x 90 0.143 ->
-// 0.125 ms, 512 x 512 0.488 -> 0.458, the adjoint of 256 x 256, 8 spp 2.00 -> 1.94. With an early
-// trigger, the next launch's CTAs waiting on the chip: 0.127, 0.466, 1.94.
-template <typename... Params, typename... Args>
-cudaError_t launch(void (*kernel)(Params...), uint32_t grid, cudaStream_t stream, Args... args)
+// A chained launch (launch.cuh). Measured against plain ones (one B200): 160 x 90 0.143 -> 0.125 ms,
+// 512 x 512 0.488 -> 0.458, the adjoint of 256 x 256, 8 spp 2.00 -> 1.94. With an early trigger, the
+// next launch's CTAs waiting on the chip: 0.127, 0.466, 1.94.
+template <typename Kernel, typename... Args>
+cudaError_t launch(Kernel kernel, uint32_t grid, cudaStream_t stream, Args... args)
 {
-    cudaLaunchAttribute early;
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(grid);
-    config.blockDim = dim3(kWaveThreads);
-    config.stream = stream;
-    config.attrs = &early;
-    config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+    return launch_chained(kernel, grid, kWaveThreads, 0, stream, args...);
 }
 
 // Every sub-wave of every wave of the plan, its shade kernels in mode kMode with kMinBlocks CTAs
