@@ -65,6 +65,13 @@ CaelixResult upload_materials(CaelixScene* scene, cudaStream_t stream, bool* cod
     if (!scene->materials_dirty) return CAELIX_OK;
     std::vector<uint32_t> codes;
     cx::light_code_set(scene->materials, scene->encoding, scene->light_options.min_emission, codes);
+    uint32_t blocks = 0;
+    const cx::Encoding enc = cx::encoding_of(scene->encoding);
+    for (uint32_t v = 0; v < cx::kMaterialCodes; ++v) {
+        const uint32_t c = cx::material_code(v, enc);
+        blocks |= ((codes[c >> 5] >> (c & 31u)) & 1u) << (v >> cx::kLightBlockShift);
+    }
+    codes.push_back(blocks);
     *codes_changed = codes != scene->light_codes;
     std::vector<float> table;
     cx::pack_materials(scene->materials, scene->encoding, table);

@@ -170,9 +170,10 @@ struct FinalizeArgs
     const uint16_t* voxels;
     uint32_t n;
     uint32_t group_shift;
-    const uint4* slots;
-    uint32_t capacity;
-    uint32_t max_probe;
+    CellGrid cells;
+    const float* power;
+    const uint32_t* light_codes;
+    uint8_t* light_flag;  // nullptr: no lights
     uint32_t* records;
     const uint32_t* list;        // nullptr: every brick; else the bricks list[0 .. *list_count)
     const uint32_t* list_count;
@@ -229,6 +230,22 @@ __device__ __forceinline__ uint32_t opaque_byte(const uint4& v)
     return b;
 }
 
+// The bits of 8 values that are neither air nor opaque (bit j = value j).
+template <uint32_t kEnc>
+__device__ __forceinline__ uint32_t other_byte(const uint4& v)
+{
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t b = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t clear = ~opaque_top<kEnc>(w[i]) & 0x80008000u;
+        const uint32_t low = w[i] & 0x7FFF7FFFu;
+        const uint32_t other = clear & (low + 0x7FFF7FFFu);  // (a clear value has no bit 15 of its own)
+        b |= (((other >> 15) & 1u) | ((other >> 30) & 2u)) << (2 * i);
+    }
+    return b;
+}
+
 // The light bits of 8 values (bit j = value j's material code is in the light code set).
 template <uint32_t kEnc>
 __device__ __forceinline__ uint32_t light_byte(const uint4& v, const uint32_t* __restrict__ codes)
@@ -241,6 +258,17 @@ __device__ __forceinline__ uint32_t light_byte(const uint4& v, const uint32_t* _
         const uint32_t c = material_code((w[i >> 1] >> (16 * (i & 1))) & 0xFFFFu, E);
         b |= ((__ldg(codes + (c >> 5)) >> (c & 31)) & 1u) << i;
     }
+    return b;
+}
+
+// Bit 0: one of 8 values is in a block of 2,048 raw values that holds a light voxel's value (the last word
+// of the light code set).
+__device__ __forceinline__ uint32_t light_block_bits(const uint4& v, uint32_t blocks)
+{
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t b = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b |= (blocks >> ((w[i] >> 11) & 31u)) | (blocks >> (w[i] >> 27));
     return b;
 }
 
@@ -262,8 +290,8 @@ struct BrickFaces
 };
 
 __device__ __forceinline__ BrickFaces load_brick_faces(const int32_t* __restrict__ keys,
-                                                       const uint16_t* __restrict__ voxels, const uint4* slots,
-                                                       uint32_t capacity, uint32_t max_probe, uint32_t b, uint32_t lane)
+                                                       const uint16_t* __restrict__ voxels, const CellGrid& cells,
+                                                       uint32_t b, uint32_t lane)
 {
     BrickFaces f;
     const int32_t bx = __ldg(keys + 3ull * b), by = __ldg(keys + 3ull * b + 1), bz = __ldg(keys + 3ull * b + 2);
@@ -275,7 +303,7 @@ __device__ __forceinline__ BrickFaces load_brick_faces(const int32_t* __restrict
         const int dx = lane == 0 ? 1 : (lane == 1 ? -1 : 0);
         const int dy = lane == 2 ? 1 : (lane == 3 ? -1 : 0);
         const int dz = lane == 4 ? 1 : (lane == 5 ? -1 : 0);
-        my_nbr = hash_lookup(slots, capacity, max_probe, bx + dx, by + dy, bz + dz);
+        my_nbr = brick_record(cells, bx + dx, by + dy, bz + dz);
     }
     const uint32_t fj = lane & 7u, fg = lane >> 3;
     const uint32_t nx_pos = __shfl_sync(0xFFFFFFFFu, my_nbr, 0);
@@ -314,17 +342,17 @@ __device__ __forceinline__ uint32_t mask_word(uint32_t b0, uint32_t b1, uint32_t
     return o;
 }
 
-template <uint32_t kEnc>
-__device__ __forceinline__ OpaqueMasks opaque_masks(const BrickFaces& f, uint32_t lane)
+// The masks of a property of values, from its bits of the brick's values (b0, b1: a byte per lane, as
+// for mask_word), of the y and z faces' rows (fb) and of the x faces' values (as in BrickFaces).
+__device__ __forceinline__ OpaqueMasks value_masks(uint32_t b0, uint32_t b1, uint32_t fb, bool xp0, bool xn0, bool xp1,
+                                                   bool xn1, uint32_t lane)
 {
-    constexpr uint32_t kOpaque = encoding_of(kEnc).opaque_mask;
     const uint32_t kz = (lane >> 1) & 7u, kyh = lane & 1u;
-    const uint32_t o = mask_word(opaque_byte<kEnc>(f.v0), opaque_byte<kEnc>(f.v1), lane);
-    const uint32_t fxp0 = __ballot_sync(0xFFFFFFFFu, f.xf[0] & kOpaque);
-    const uint32_t fxn0 = __ballot_sync(0xFFFFFFFFu, f.xf[1] & kOpaque);
-    const uint32_t fxp1 = __ballot_sync(0xFFFFFFFFu, f.xf[2] & kOpaque);
-    const uint32_t fxn1 = __ballot_sync(0xFFFFFFFFu, f.xf[3] & kOpaque);
-    const uint32_t fb = opaque_byte<kEnc>(f.fv);
+    const uint32_t o = mask_word(b0, b1, lane);
+    const uint32_t fxp0 = __ballot_sync(0xFFFFFFFFu, xp0);
+    const uint32_t fxn0 = __ballot_sync(0xFFFFFFFFu, xn0);
+    const uint32_t fxp1 = __ballot_sync(0xFFFFFFFFu, xp1);
+    const uint32_t fxn1 = __ballot_sync(0xFFFFFFFFu, xn1);
     const uint32_t fyp = __shfl_sync(0xFFFFFFFFu, fb, kz), fyn = __shfl_sync(0xFFFFFFFFu, fb, 8 + kz);
     uint32_t fzp = 0, fzn = 0;
 #pragma unroll
@@ -349,7 +377,15 @@ __device__ __forceinline__ OpaqueMasks opaque_masks(const BrickFaces& f, uint32_
 }
 
 template <uint32_t kEnc>
-__global__ void __launch_bounds__(kFinalizeWarps * 32, 6) finalize_kernel(const FinalizeArgs a)
+__device__ __forceinline__ OpaqueMasks opaque_masks(const BrickFaces& f, uint32_t lane)
+{
+    constexpr uint32_t kOpaque = encoding_of(kEnc).opaque_mask;
+    return value_masks(opaque_byte<kEnc>(f.v0), opaque_byte<kEnc>(f.v1), opaque_byte<kEnc>(f.fv), (f.xf[0] & kOpaque) != 0,
+                       (f.xf[1] & kOpaque) != 0, (f.xf[2] & kOpaque) != 0, (f.xf[3] & kOpaque) != 0, lane);
+}
+
+template <uint32_t kEnc>
+__global__ void __launch_bounds__(kFinalizeWarps * 32, 4) finalize_kernel(const FinalizeArgs a)
 {
     constexpr Encoding E = encoding_of(kEnc);
     __shared__ __align__(16) uint32_t s_stage[kFinalizeWarps][kFinalizeStageWords];
@@ -357,13 +393,15 @@ __global__ void __launch_bounds__(kFinalizeWarps * 32, 6) finalize_kernel(const 
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint16_t* vox = reinterpret_cast<uint16_t*>(s_stage[warp]);  // [512] then faces [6][64]
     uint16_t* rec16 = reinterpret_cast<uint16_t*>(s_record[warp]);
-    const uint32_t x = lane & 7u, ylo = lane >> 3;
+    __shared__ uint16_t s_list[kFinalizeWarps][kBrickVoxels];  // the voxels under the per-voxel rules
+    __shared__ uint32_t s_occ[kFinalizeWarps][16];
     const uint32_t fj = lane & 7u, fg = lane >> 3;  // face loads: row fj of face 2 + fg
     const uint32_t items = a.list ? *a.list_count : a.n;
+    const uint32_t light_blocks = a.light_flag ? __ldg(a.light_codes + kLightCodeWords) : 0u;
     for (uint32_t item = blockIdx.x * kFinalizeWarps + warp; item < items; item += gridDim.x * kFinalizeWarps) {
         const uint32_t b = a.list ? __ldg(a.list + item) : item;
         const int32_t bx = __ldg(a.keys + 3ull * b), by = __ldg(a.keys + 3ull * b + 1), bz = __ldg(a.keys + 3ull * b + 2);
-        const BrickFaces bf = load_brick_faces(a.keys, a.voxels, a.slots, a.capacity, a.max_probe, b, lane);
+        const BrickFaces bf = load_brick_faces(a.keys, a.voxels, a.cells, b, lane);
         const uint4 v0 = bf.v0, v1 = bf.v1, fv = bf.fv;
         const uint32_t* xf = bf.xf;
         __syncwarp();  // the previous brick's reads of the staging are done
@@ -376,10 +414,23 @@ __global__ void __launch_bounds__(kFinalizeWarps * 32, 6) finalize_kernel(const 
             vox[512 + 64 + lane + 32 * h] = (uint16_t)xf[2 * h + 1];
         }
         __syncwarp();
+        if (a.light_flag && __ldg(a.power + b) > 0.0f) {
+            // First by the blocks of values that hold light codes: sixteen lookups per lane are a quarter of
+            // the instructions of a brick.
+            bool any = __any_sync(0xFFFFFFFFu, (light_block_bits(v0, light_blocks) | light_block_bits(v1, light_blocks)) & 1u);
+            if (any)
+                any = __any_sync(0xFFFFFFFFu, (light_byte<kEnc>(v0, a.light_codes) | light_byte<kEnc>(v1, a.light_codes)) != 0u);
+            if (lane == 0) a.light_flag[b] = any ? 1 : 0;
+        } else if (a.light_flag && lane == 0) {
+            a.light_flag[b] = 0;
+        }
         // A clean brick (every value of it and of its six neighbour faces air or opaque) keeps
         // its raw values as the payload, and a voxel of it is occupied iff it is opaque and not
-        // all six of its neighbours are: shifted masks of the opaque voxels. Other bricks take
-        // the per-voxel rules.
+        // all six of its neighbours are: shifted masks of the opaque voxels. In other bricks that
+        // holds for the opaque voxels and for air without a non-opaque value beside it; the per-voxel
+        // rules run for the non-opaque values and the air beside them, which the same masks of those
+        // values list (with one such voxel in 64 the rules over every voxel took 222 us over 100 k
+        // bricks, all issue; 131 now, the light flags included).
         const bool dirty =
             __any_sync(0xFFFFFFFFu, impure<kEnc>(v0) || impure<kEnc>(v1) || impure<kEnc>(fv) || impure16<kEnc>(xf[0]) ||
                                         impure16<kEnc>(xf[1]) || impure16<kEnc>(xf[2]) || impure16<kEnc>(xf[3]));
@@ -387,16 +438,34 @@ __global__ void __launch_bounds__(kFinalizeWarps * 32, 6) finalize_kernel(const 
         // y = 4 (k & 1) + (0 .. 3) at z = k >> 1.
         uint32_t my_occ = 0;
         const uint32_t kz = (lane >> 1) & 7u, kyh = lane & 1u;
-        if (!dirty) {
-            const OpaqueMasks m = opaque_masks<kEnc>(bf, lane);
-            my_occ = m.o & ~(m.n[0] & m.n[1] & m.n[2] & m.n[3] & m.n[4] & m.n[5]);
-        } else {
-#pragma unroll 2
-            for (uint32_t k = 0; k < 16; ++k) {
-                const uint32_t y = ylo + 4 * (k & 1), z = k >> 1;
-                const uint32_t vi = lane + 32 * k;
-                const uint32_t raw = vox[vi];
-                const uint32_t v = material_code(raw, E);
+        const OpaqueMasks m = opaque_masks<kEnc>(bf, lane);
+        my_occ = m.o & ~(m.n[0] & m.n[1] & m.n[2] & m.n[3] & m.n[4] & m.n[5]);
+        if (dirty) {
+            // The raw values (opaque voxels and air keep them), then the listed voxels' results over them.
+            uint2* pay = reinterpret_cast<uint2*>(s_record[warp]) + kRecordPayloadWord / 2;
+            pay[2 * lane] = make_uint2(v0.x, v0.y);
+            pay[2 * lane + 1] = make_uint2(v0.z, v0.w);
+            pay[64 + 2 * lane] = make_uint2(v1.x, v1.y);
+            pay[64 + 2 * lane + 1] = make_uint2(v1.z, v1.w);
+            const OpaqueMasks t = value_masks(other_byte<kEnc>(v0), other_byte<kEnc>(v1), other_byte<kEnc>(fv),
+                                              impure16<kEnc>(xf[0]), impure16<kEnc>(xf[1]), impure16<kEnc>(xf[2]),
+                                              impure16<kEnc>(xf[3]), lane);
+            uint32_t listed = lane < 16 ? (t.o | (~m.o & (t.n[0] | t.n[1] | t.n[2] | t.n[3] | t.n[4] | t.n[5]))) : 0u;
+            const uint32_t mine = (uint32_t)__popc(listed);
+            const uint32_t upto = warp_inclusive_sum(mine);
+            const uint32_t count = __shfl_sync(0xFFFFFFFFu, upto, 31);
+            uint16_t* out = s_list[warp] + (upto - mine);
+            while (listed) {
+                const uint32_t bit = (uint32_t)__ffs(listed) - 1u;
+                listed &= listed - 1u;
+                *out++ = (uint16_t)(32u * lane + bit);
+            }
+            if (lane < 16) s_occ[warp][lane] = my_occ;
+            __syncwarp();
+            for (uint32_t j = lane; j < count; j += 32) {
+                const uint32_t vi = s_list[warp][j];
+                const uint32_t x = vi & 7u, y = (vi >> 3) & 7u, z = vi >> 6;
+                const uint32_t v = material_code(vox[vi], E);
                 uint32_t nb[6];
                 nb[0] = vox[x < 7 ? vi + 1 : 512 + 0 * 64 + y + 8 * z];
                 nb[1] = vox[x > 0 ? vi - 1 : 512 + 1 * 64 + y + 8 * z];
@@ -411,12 +480,12 @@ __global__ void __launch_bounds__(kFinalizeWarps * 32, 6) finalize_kernel(const 
                     opaque_count += nop ? 1u : 0u;
                     if (!nop && (nb[d] & E.id_mask) != v) faces |= 1u << d;
                 }
-                const uint32_t result = (v & E.opaque_mask) ? v : (v | (faces << E.face_shift));
-                const bool iface = (v & E.opaque_mask) != 0 || faces != 0;
+                const uint32_t result = v | (faces << E.face_shift);  // (a listed voxel is not opaque)
                 rec16[2 * kRecordPayloadWord + vi] = (uint16_t)result;
-                const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, opaque_count < 6 && result != 0 && iface);
-                if (lane == k) my_occ = ballot;
+                if (opaque_count < 6 && result != 0 && faces != 0) atomicOr(&s_occ[warp][vi >> 5], 1u << (vi & 31u));
             }
+            __syncwarp();
+            if (lane < 16) my_occ = s_occ[warp][lane];
         }
         // Occupancy word w = 2 cell + half of coarse cell c = (x >> 2) + 2 (y >> 2) + 4 (z >> 2),
         // bit (x & 3) + 4 (y & 3) + 16 (z & 3) - 32 half: the lanes of even z join the next z.
@@ -480,33 +549,21 @@ struct LightArgs
     uint32_t group_shift;
     uint32_t groups[3];
     int32_t origin[3];
-    const uint4* slots;
-    uint32_t capacity;
-    uint32_t max_probe;
+    CellGrid cells;
+    const uint8_t* light_flag;
     const float4* materials;
     const uint32_t* light_codes;
 };
 
-// A brick with power above 0 and a voxel whose code is a light code is a light brick. A warp takes
-// 32 consecutive bricks: each lane reads one brick's power, then the warp reads the values of each
-// brick with power (two 16-byte words per lane) and appends the light bricks with one atomic.
-template <uint32_t kEnc>
+// A brick with power above 0 and a voxel whose code is a light code (finalize_kernel's flag) is a light
+// brick: appended, one atomic per warp. The flags of bricks that a flush does not finalize again are
+// those of their unchanged values and power. (Reading the values here took 48 us over 100 k bricks with
+// power, finalize reads them anyway.)
 __global__ void light_collect_kernel(const LightArgs a, uint32_t* counter, uint32_t* lkeys, uint32_t* lbricks)
 {
-    const uint32_t first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
-    if (first >= a.n) return;
-    const uint32_t i = first + lane;
-    uint32_t todo = __ballot_sync(0xFFFFFFFFu, i < a.n && a.power[i] > 0.0f);
-    uint32_t found = 0;
-    while (todo) {
-        const uint32_t l = (uint32_t)(__ffs(todo) - 1);
-        todo &= todo - 1u;
-        const uint4* vox = reinterpret_cast<const uint4*>(a.voxels + 512ull * (first + l));
-        const uint32_t bits = light_byte<kEnc>(__ldg(vox + lane), a.light_codes) |
-                              light_byte<kEnc>(__ldg(vox + 32 + lane), a.light_codes);
-        if (__any_sync(0xFFFFFFFFu, bits != 0u)) found |= 1u << l;
-    }
+    const uint32_t found = __ballot_sync(0xFFFFFFFFu, i < a.n && a.light_flag[i] != 0);
     if (!found) return;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(counter, (uint32_t)__popc(found));
@@ -586,7 +643,7 @@ __global__ void __launch_bounds__(kLightWarps * 32) light_measure_kernel(const L
         }
         return;
     }
-    const BrickFaces bf = load_brick_faces(a.keys, a.voxels, a.slots, a.capacity, a.max_probe, lbricks[k], lane);
+    const BrickFaces bf = load_brick_faces(a.keys, a.voxels, a.cells, lbricks[k], lane);
     uint32_t open[6];
     light_open_masks<kEnc>(bf, a.light_codes, lane, open);
     uint32_t total = 0;
@@ -683,7 +740,7 @@ __global__ void __launch_bounds__(kLightWarps * 32) light_write_kernel(const Lig
             hp[2] = src[2];
         }
     } else {
-        const BrickFaces bf = load_brick_faces(a.keys, a.voxels, a.slots, a.capacity, a.max_probe, b, lane);
+        const BrickFaces bf = load_brick_faces(a.keys, a.voxels, a.cells, b, lane);
         s_vox[warp][lane] = bf.v0;
         s_vox[warp][32 + lane] = bf.v1;
         __syncwarp();
@@ -833,8 +890,12 @@ __global__ void group_occupancy_kernel(const int32_t* __restrict__ keys, uint32_
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    // One lane per run of bricks of one group (neighbours in linear order mostly share it): a thread per
+    // brick asking the flag's word took 31 us over 100 k bricks of 72 groups.
     const uint32_t g = brick_group(keys, i, gg.origin, gg.groups, gg.shift);
-    if (!(flags[g] & kGroupOccupied)) atomicOr(&flags[g], kGroupOccupied);
+    const uint32_t peers = __match_any_sync(__activemask(), g);
+    if ((threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1u && !(flags[g] & kGroupOccupied))
+        atomicOr(&flags[g], kGroupOccupied);
 }
 
 __global__ void group_touch_kernel(const int32_t* __restrict__ keys, uint32_t n, const uint32_t* __restrict__ marks,
@@ -937,6 +998,11 @@ bool scene_grid(const int32_t key_min[3], const int32_t key_max[3], uint32_t gro
         if (cells > (1ull << 32)) return false;
     }
     return true;
+}
+
+CellGrid cell_grid(const DeviceScene& s)
+{
+    return CellGrid{s.cells, {s.origin[0], s.origin[1], s.origin[2]}, {s.grid[0], s.grid[1], s.grid[2]}};
 }
 
 SceneView scene_view(const DeviceScene& s)
@@ -1060,7 +1126,7 @@ static BuildScratch build_scratch(const DeviceScene& s)
 void scene_release(DeviceScene& s)
 {
     void* ptrs[] = {s.keys,          s.voxels,       s.power,        s.records,       s.hash_slots,
-                    s.bitmap,        s.cells,        s.heap,         s.group_rows,    s.frames,
+                    s.bitmap,        s.cells,        s.light_flag,        s.heap,         s.group_rows,    s.frames,
                     s.light_headers, s.light_group,  s.light_entry,  s.light_brick,   s.scratch,
                     s.tree_memory,   s.status,       s.heap_prev,    s.unit_of_brick, s.unit_of_brick_prev,
                     s.group_gen,     s.group_flag};
@@ -1082,6 +1148,13 @@ cudaError_t scene_alloc_inputs(DeviceScene& s, uint32_t n, cudaStream_t stream)
 }
 
 namespace {
+
+FinalizeArgs finalize_args(const DeviceScene& s, const uint32_t* list, const uint32_t* list_count)
+{
+    return FinalizeArgs{s.keys,  s.voxels,      s.brick_count,                     s.group_shift, cell_grid(s),
+                        s.power, s.light_codes, s.lights ? s.light_flag : nullptr, s.records,     list,
+                        list_count};
+}
 
 void launch_finalize(const FinalizeArgs& fa, uint32_t encoding, uint32_t items, cudaStream_t stream)
 {
@@ -1150,25 +1223,26 @@ cudaError_t scene_build_device(DeviceScene& s, const int32_t origin[3], const ui
     if (n > 0)
         cell_table_kernel<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(s.keys, n, origin[0], origin[1], origin[2],
                                                                              grid[0], grid[1], s.bitmap, s.cells);
-    CX_TRY(cudaMemcpyAsync(&s.hash_max_probe, d_max_probe, 4, cudaMemcpyDeviceToHost, stream));
-    CX_TRY(cudaStreamSynchronize(stream));
+    // (Read by the time scene_build_lights returns: it waits for the stream.)
+    CX_TRY(cudaMemcpyAsync(s.pinned + 5, d_max_probe, 4, cudaMemcpyDeviceToHost, stream));
 
     // Records.
     CX_TRY(alloc(s.records, s.capacity.records, (uint64_t)kRecordWords * n));
+    CX_TRY(alloc(s.light_flag, s.capacity.light_flag, n));
     if (n > 0) {
-        FinalizeArgs fa{s.keys,  s.voxels,          n,         group_shift, s.hash_slots, s.hash_capacity,
-                        s.hash_max_probe, s.records, nullptr, nullptr};
+        const FinalizeArgs fa = finalize_args(s, nullptr, nullptr);
         launch_finalize(fa, s.encoding, n, stream);
     }
-    return scene_build_lights(s, stream, device_status_out);
+    CX_TRY(scene_build_lights(s, stream, device_status_out));
+    s.hash_max_probe = s.pinned[5];
+    return cudaSuccess;
 }
 
 cudaError_t scene_refinalize(DeviceScene& s, const uint32_t* list, const uint32_t* list_count, uint32_t max_count,
                              cudaStream_t stream)
 {
     if (max_count == 0) return cudaSuccess;
-    FinalizeArgs fa{s.keys,  s.voxels,          s.brick_count, s.group_shift, s.hash_slots, s.hash_capacity,
-                    s.hash_max_probe, s.records, list,       list_count};
+    const FinalizeArgs fa = finalize_args(s, list, list_count);
     launch_finalize(fa, s.encoding, max_count, stream);
     return cudaGetLastError();
 }
@@ -1254,9 +1328,8 @@ cudaError_t scene_build_lights(DeviceScene& s, cudaStream_t stream, uint32_t* de
                  group_shift,
                  {s.groups[0], s.groups[1], s.groups[2]},
                  {s.origin[0], s.origin[1], s.origin[2]},
-                 s.hash_slots,
-                 s.hash_capacity,
-                 s.hash_max_probe,
+                 cell_grid(s),
+                 s.light_flag,
                  s.materials,
                  s.light_codes};
     uint32_t* d_light_count = s.status + 5;
@@ -1265,12 +1338,7 @@ cudaError_t scene_build_lights(DeviceScene& s, cudaStream_t stream, uint32_t* de
     uint32_t* lkeys_alt = bs.home_alt;
     uint32_t* lbricks_alt = bs.order_alt;
     if (n > 0 && s.lights) {
-        if (packed)
-            light_collect_kernel<kEncodingPacked>
-                <<<blocks_for(n, kThreads), kThreads, 0, stream>>>(la, d_light_count, lkeys, lbricks);
-        else
-            light_collect_kernel<kEncodingBlockId>
-                <<<blocks_for(n, kThreads), kThreads, 0, stream>>>(la, d_light_count, lkeys, lbricks);
+        light_collect_kernel<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(la, d_light_count, lkeys, lbricks);
     }
     CX_TRY(cudaMemcpyAsync(s.pinned, d_light_count, 4, cudaMemcpyDeviceToHost, stream));
     CX_TRY(cudaStreamSynchronize(stream));

@@ -41,6 +41,9 @@ __host__ __device__ __forceinline__ uint32_t material_code(uint32_t v, const Enc
 // the scene's min_emission.
 constexpr uint32_t kMaterialCodes = 65536;
 constexpr uint32_t kLightCodeWords = kMaterialCodes / 32;
+// On the device one more word follows: bit t set when a raw block value in [2048 t, 2048 (t + 1)) has a
+// light code.
+constexpr uint32_t kLightBlockShift = 11;
 
 struct EntityView;
 
@@ -146,6 +149,7 @@ struct DeviceScene
     uint32_t* records = nullptr;
     uint4* hash_slots = nullptr;
     uint32_t* bitmap = nullptr;
+    uint8_t* light_flag = nullptr;  // per brick, by finalize: power above 0 and a voxel of a light code
     uint2* cells = nullptr;  // the bitmap's words, each with the record of its first brick (cell_table_kernel)
     uint32_t* heap = nullptr;
     uint32_t* group_rows = nullptr;
@@ -185,7 +189,7 @@ struct DeviceScene
     // Element capacities of the buffers above: a rebuild reallocates a buffer only to grow it.
     struct
     {
-        uint64_t keys, voxels, power, scratch, hash_slots, bitmap, cells, records, group_rows, light_headers,
+        uint64_t keys, voxels, power, scratch, hash_slots, bitmap, cells, light_flag, records, group_rows, light_headers,
             light_group, light_entry, light_brick, frames, heap, heap_prev, unit_of_brick, unit_of_brick_prev, group_gen,
             group_flag;
     } capacity{};
@@ -263,5 +267,7 @@ cudaError_t scene_build_light_tree(const DeviceScene& s, cudaStream_t stream, ui
 cudaError_t scene_read_status(const DeviceScene& s, cudaStream_t stream, uint32_t* device_status_out);
 void scene_release(DeviceScene& s);
 SceneView scene_view(const DeviceScene& s);
+struct CellGrid;
+CellGrid cell_grid(const DeviceScene& s);
 
 }  // namespace cx

@@ -69,4 +69,21 @@ __device__ __forceinline__ uint32_t cell_record(const uint2 word, uint32_t lin)
     return word.y + (uint32_t)__popc(word.x & ((1u << (lin & 31u)) - 1u));
 }
 
+// The cell table with its grid, for lookups by brick key.
+struct CellGrid
+{
+    const uint2* cells;
+    int32_t origin[3];
+    uint32_t grid[3];
+};
+// The record of brick (x, y, z), or 0xFFFFFFFF.
+__device__ __forceinline__ uint32_t brick_record(const CellGrid& g, int32_t x, int32_t y, int32_t z)
+{
+    const uint32_t cx = (uint32_t)(x - g.origin[0]), cy = (uint32_t)(y - g.origin[1]), cz = (uint32_t)(z - g.origin[2]);
+    if (cx >= g.grid[0] || cy >= g.grid[1] || cz >= g.grid[2]) return 0xFFFFFFFFu;
+    const uint32_t lin = cx + g.grid[0] * (cy + g.grid[1] * cz);  // (the grid has at most 2^32 cells)
+    uint2 word;
+    return cell_occupied(g.cells, lin, word) ? cell_record(word, lin) : 0xFFFFFFFFu;
+}
+
 }  // namespace cx

@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(kStageThreads)
     staging_update_kernel(const uint4* __restrict__ stage_voxels, const uint32_t* __restrict__ slots,
                           const float* __restrict__ slot_power, uint32_t count,
                           const uint32_t* __restrict__ record_of_slot, const int32_t* __restrict__ keys,
-                          uint4* __restrict__ voxels, float* __restrict__ power, const uint4* __restrict__ hash_slots,
-                          uint32_t hash_capacity, uint32_t hash_max_probe, uint32_t* __restrict__ marks,
+                          uint4* __restrict__ voxels, float* __restrict__ power, const CellGrid cells,
+                          uint32_t* __restrict__ marks,
                           uint32_t epoch, uint32_t* __restrict__ list, uint32_t* __restrict__ list_count)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -92,8 +92,7 @@ __global__ void __launch_bounds__(kStageThreads)
         const int dx = lane == 0 ? 1 : (lane == 1 ? -1 : 0);
         const int dy = lane == 2 ? 1 : (lane == 3 ? -1 : 0);
         const int dz = lane == 4 ? 1 : (lane == 5 ? -1 : 0);
-        target = hash_lookup(hash_slots, hash_capacity, hash_max_probe, keys[3ull * r] + dx, keys[3ull * r + 1] + dy,
-                             keys[3ull * r + 2] + dz);
+        target = brick_record(cells, keys[3ull * r] + dx, keys[3ull * r + 1] + dy, keys[3ull * r + 2] + dz);
     }
     if (target != 0xFFFFFFFFu && atomicExch(marks + target, epoch) != epoch)
         list[atomicAdd(list_count, 1u)] = target;
@@ -159,7 +158,7 @@ cudaError_t staging_update(const uint16_t* stage_voxels, const uint32_t* slots, 
     if (count == 0) return cudaSuccess;
     staging_update_kernel<<<blocks(32ull * count), kStageThreads, 0, stream>>>(
         reinterpret_cast<const uint4*>(stage_voxels), slots, power, count, record_of_slot, s.keys,
-        reinterpret_cast<uint4*>(s.voxels), s.power, s.hash_slots, s.hash_capacity, s.hash_max_probe, marks, epoch,
+        reinterpret_cast<uint4*>(s.voxels), s.power, cell_grid(s), marks, epoch,
         list, list_count);
     return cudaGetLastError();
 }
