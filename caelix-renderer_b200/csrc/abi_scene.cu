@@ -30,6 +30,9 @@ bool key_ok(const CaelixBrickKey& k)
            k.z < kKeyLimit;
 }
 
+// Keys whose place in the slot map is asked for ahead of their lookup.
+constexpr uint32_t kKeyLookahead = 16;
+
 // 21 bits per axis (the key moved to [0, 2^21)).
 uint64_t pack_key(const CaelixBrickKey& k)
 {
@@ -49,11 +52,24 @@ void key_bounds(CaelixScene* scene)
         scene->key_min[a] = n ? scene->keys[a] : 0;
         scene->key_max[a] = n ? scene->keys[a] : 0;
     }
-    for (size_t slot = 1; slot < n; ++slot)
-        for (int a = 0; a < 3; ++a) {
-            scene->key_min[a] = std::min(scene->key_min[a], scene->keys[3 * slot + a]);
-            scene->key_max[a] = std::max(scene->key_max[a], scene->keys[3 * slot + a]);
+    // Four keys at a time, so that the loop is one of twelve independent lanes.
+    const int32_t* k = scene->keys.data();
+    int32_t lo[12], hi[12];
+    for (int j = 0; j < 12; ++j) lo[j] = hi[j] = n ? k[j % 3] : 0;
+    for (size_t slot = 0; slot + 4 <= n; slot += 4)
+        for (int j = 0; j < 12; ++j) {
+            lo[j] = std::min(lo[j], k[3 * slot + j]);
+            hi[j] = std::max(hi[j], k[3 * slot + j]);
         }
+    for (size_t slot = n - n % 4; slot < n; ++slot)
+        for (int j = 0; j < 3; ++j) {
+            lo[j] = std::min(lo[j], k[3 * slot + j]);
+            hi[j] = std::max(hi[j], k[3 * slot + j]);
+        }
+    for (int j = 0; j < 12; ++j) {
+        scene->key_min[j % 3] = std::min(scene->key_min[j % 3], lo[j]);
+        scene->key_max[j % 3] = std::max(scene->key_max[j % 3], hi[j]);
+    }
 }
 
 // The device form of a scene's material table and its light code set, after a change of either
@@ -584,10 +600,11 @@ CAELIX_API CaelixResult caelix_scene_upload_bricks(CaelixScene* scene, uint32_t 
     std::vector<std::pair<uint64_t, float>> taken_power;
     std::vector<uint32_t> slot(count);
     for (uint32_t i = 0; i < count; ++i) {
+        if (i + kKeyLookahead < count) scene->slot_of.prefetch(pack_key(keys[i + kKeyLookahead]));
         const uint64_t packed = pack_key(keys[i]);
-        const auto ins = scene->slot_of.emplace(packed, (uint32_t)scene->slot_power.size());
-        slot[i] = ins.first->second;
-        if (ins.second) {
+        bool added = false;
+        slot[i] = scene->slot_of.insert(packed, (uint32_t)scene->slot_power.size(), &added);
+        if (added) {
             const int32_t k3[3] = {keys[i].x, keys[i].y, keys[i].z};
             const bool first = scene->slot_power.empty();
             scene->keys.insert(scene->keys.end(), {k3[0], k3[1], k3[2]});
@@ -707,35 +724,35 @@ CAELIX_API CaelixResult caelix_scene_remove_bricks(CaelixScene* scene, uint32_t 
     // host state changes only after the moves have been checked.
     const uint32_t old_slots = (uint32_t)scene->slot_power.size();
     uint32_t n = old_slots;
-    std::unordered_map<uint32_t, uint32_t> source;
-    std::unordered_map<uint64_t, uint32_t> moved;
-    std::unordered_map<uint64_t, uint32_t> gone;
+    KeyMap source, moved, gone;  // (source: by slot)
     auto original = [&](uint32_t slot) {
-        const auto m = source.find(slot);
-        return m != source.end() ? m->second : slot;
+        const uint32_t* m = source.find(slot);
+        return m ? *m : slot;
     };
     auto key_of = [&](uint32_t slot) {
         const uint32_t o = original(slot);
         return pack_key(CaelixBrickKey{scene->keys[3ull * o], scene->keys[3ull * o + 1], scene->keys[3ull * o + 2]});
     };
     for (uint32_t i = 0; i < count; ++i) {
+        if (i + kKeyLookahead < count && key_ok(keys[i + kKeyLookahead]))
+            scene->slot_of.prefetch(pack_key(keys[i + kKeyLookahead]));
         if (!key_ok(keys[i])) continue;
         const uint64_t k = pack_key(keys[i]);
-        if (gone.count(k)) continue;
+        if (gone.find(k)) continue;
         uint32_t slot;
-        if (const auto m = moved.find(k); m != moved.end()) {
-            slot = m->second;
-            moved.erase(m);
-        } else if (const auto it = scene->slot_of.find(k); it != scene->slot_of.end()) {
-            slot = it->second;
+        if (const uint32_t* m = moved.find(k)) {
+            slot = *m;
+            moved.erase(k);
+        } else if (const uint32_t* known = scene->slot_of.find(k)) {
+            slot = *known;
         } else {
             continue;
         }
-        gone.emplace(k, slot);
+        gone.set(k, slot);
         const uint32_t last = n - 1;
         if (slot != last) {
-            moved[key_of(last)] = slot;
-            source[slot] = original(last);
+            moved.set(key_of(last), slot);
+            source.set(slot, original(last));
         }
         source.erase(last);
         n = last;
@@ -745,20 +762,23 @@ CAELIX_API CaelixResult caelix_scene_remove_bricks(CaelixScene* scene, uint32_t 
     // (on the host arrays and on the device) never overlap.
     std::vector<uint32_t> moves;
     moves.reserve(2 * source.size());
-    for (const auto& kv : source) {
-        if (kv.first >= n || kv.second < n || kv.second >= old_slots) {
-            log(CAELIX_LOG_ERROR, "caelix_scene_remove_bricks: bad staging move %u <- %u (nothing removed)", kv.first,
-                kv.second);
-            return CAELIX_ERROR_INVALID_ARGUMENT;
+    bool sound = true;
+    source.each([&](uint64_t to, uint32_t from) {
+        if (to >= n || from < n || from >= old_slots) {
+            if (sound)
+                log(CAELIX_LOG_ERROR, "caelix_scene_remove_bricks: bad staging move %u <- %u (nothing removed)", (uint32_t)to,
+                    from);
+            sound = false;
         }
-        moves.push_back(kv.first);
-        moves.push_back(kv.second);
-    }
-    for (const auto& kv : gone) scene->slot_of.erase(kv.first);
-    for (const auto& kv : moved) scene->slot_of[kv.first] = kv.second;
-    for (const auto& kv : source) {
-        for (int a = 0; a < 3; ++a) scene->keys[3ull * kv.first + a] = scene->keys[3ull * kv.second + a];
-        scene->slot_power[kv.first] = scene->slot_power[kv.second];
+        moves.push_back((uint32_t)to);
+        moves.push_back(from);
+    });
+    if (!sound) return CAELIX_ERROR_INVALID_ARGUMENT;
+    gone.each([&](uint64_t k, uint32_t) { scene->slot_of.erase(k); });
+    moved.each([&](uint64_t k, uint32_t to) { scene->slot_of.set(k, to); });
+    for (size_t m = 0; m < moves.size(); m += 2) {
+        for (int a = 0; a < 3; ++a) scene->keys[3ull * moves[m] + a] = scene->keys[3ull * moves[m + 1] + a];
+        scene->slot_power[moves[m]] = scene->slot_power[moves[m + 1]];
     }
     scene->keys.resize(3ull * n);
     scene->slot_power.resize(n);
@@ -869,10 +889,10 @@ CAELIX_API CaelixResult caelix_scene_set_brick_power(CaelixScene* scene, uint32_
     for (uint32_t i = 0; i < count; ++i)
         if (!key_ok(keys[i]) || !std::isfinite(power[i]) || power[i] < 0.0f) return CAELIX_ERROR_INVALID_ARGUMENT;
     for (uint32_t i = 0; i < count; ++i) {
+        if (i + kKeyLookahead < count) scene->slot_of.prefetch(pack_key(keys[i + kKeyLookahead]));
         const uint64_t packed = pack_key(keys[i]);
-        const auto it = scene->slot_of.find(packed);
-        if (it != scene->slot_of.end()) {
-            const uint32_t slot = it->second;
+        if (const uint32_t* known = scene->slot_of.find(packed)) {
+            const uint32_t slot = *known;
             scene->slot_power[slot] = power[i];
             scene->slot_dirty.resize(scene->slot_power.size(), 0);
             if (!scene->slot_dirty[slot]) {

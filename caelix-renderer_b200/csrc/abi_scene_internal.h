@@ -8,6 +8,7 @@
 
 #include "../../include/caelix_b200.h"
 #include "abi_internal.h"
+#include "key_map.h"
 #include "scene.cuh"
 #include "trace.cuh"
 
@@ -45,7 +46,7 @@ struct CaelixScene
     // Brick staging. Slot s holds the brick keys[3s .. 3s+2]; its 512 block values stay on the
     // device (stage_voxels[512s ..], copied there by the upload that wrote them), its key in
     // stage_keys[3s ..] and its power in slot_power[s].
-    std::unordered_map<uint64_t, uint32_t> slot_of;
+    KeyMap slot_of;
     std::vector<int32_t> keys;
     std::vector<float> slot_power;
     std::unordered_map<uint64_t, float> pending_power;  // power of keys not uploaded yet (default 1)
