@@ -134,6 +134,7 @@ struct WavePlan
     std::vector<uint32_t> samples;   // per wave: sample indices
     std::vector<uint32_t> items;     // per wave: items
     std::vector<uint32_t> bounces;   // per wave: the largest bounce count of its views
+    bool one_view = false;
     uint32_t largest() const;        // the items of the largest wave
 };
 constexpr uint32_t kWaveMergeSlots = 1u << 23;

@@ -37,20 +37,46 @@ constexpr uint32_t kFlagShadow = 1u << 9;     // a shadow ray of the last vertex
 constexpr uint32_t kFlagExt = 1u << 10;       // an extension ray was queued
 constexpr uint32_t kFlagPrimary = 1u << 11;   // that extension ray is the camera ray
 constexpr uint32_t kLampEnds = 1u << 31;      // of a lampq entry: the path ends with this emission
-// Words of WaveBuffers::counts: 0..3 the queue lengths of the two parities (rays, paths), then
+// The counters in WaveBuffers::counts: 0..3 the queue lengths of the two parities (rays, paths), then
 // the trace and shade launches' fetch counters of the two parities, the lengths of the light draw
-// and lamp queues and the light launch's fetch counter (cleared by the next trace launch).
+// and lamp queues and the light launch's fetch counter (cleared by the next trace launch). Each has a
+// 128-byte line of its own: an atomic takes about a nanosecond at its address, and a launch over 8 M
+// paths made a million of them side by side. With lines of their own, appends of 128 entries at a time,
+// chunks of up to 256 items and rays counted per warp (one B200, 1920 x 1080 x 4 spp on 300 k bricks): the
+// first shade launch 731 -> 236 us, all of them 2.25 -> 0.94 ms, the camera rays' generation 394 -> 71 us, the
+// frame 12.1 -> 11.1 ms; 512 x 512 0.456 -> 0.424, 160 x 90 0.125 -> 0.117, 12 batched views 5.23 -> 4.72.
 constexpr uint32_t kFetchTrace = 4, kFetchShade = 6, kCountNee = 8, kCountLamp = 9, kFetchLight = 10;
-constexpr uint32_t kCountWords = 16;
-
-// The next 32-item chunk of a queue for the calling warp, from a fetch counter. A warp that is done
-// with its chunk takes the next one, so the work of a launch whose items' costs differ widely
-// spreads over the warps until its end. Every lane calls.
-__device__ __forceinline__ uint32_t fetch_chunk(uint32_t* counter)
+constexpr uint32_t kCounters = 11;
+constexpr uint32_t kCounterStride = 32;
+constexpr uint32_t kCountWords = kCounters * kCounterStride;
+__device__ __forceinline__ uint32_t* counter_of(const WaveBuffers& b, uint32_t k) { return b.counts + k * kCounterStride; }
+__device__ __forceinline__ uint32_t count_of(const WaveBuffers& b, uint32_t k)
 {
-    uint32_t base = 0;
-    if ((threadIdx.x & 31u) == 0) base = atomicAdd(counter, 32u);
-    return __shfl_sync(0xFFFFFFFFu, base, 0);
+    return *(volatile uint32_t*)counter_of(b, k);
+}
+
+// The items of a queue of n that the calling warp works on, taken `chunk` at a time from a fetch counter:
+// the work of a launch whose items' costs differ widely spreads over the warps until its end. Every lane
+// calls.
+struct WarpRange
+{
+    uint32_t at, end;
+    // Whether items [at, end) remain (a new chunk where the last one is done).
+    __device__ __forceinline__ bool more(uint32_t* counter, uint32_t n, uint32_t chunk)
+    {
+        if (at < end) return true;
+        uint32_t base = 0;
+        if ((threadIdx.x & 31u) == 0) base = atomicAdd(counter, chunk);
+        at = __shfl_sync(0xFFFFFFFFu, base, 0);
+        end = min(at + chunk, n);
+        return at < end;
+    }
+};
+// The chunk: an eighth of a warp's share of the items, in whole warps, 32 to 256.
+__device__ __forceinline__ uint32_t chunk_for(uint32_t n)
+{
+    const uint32_t share = n / (8u * gridDim.x * (blockDim.x / 32u));
+    return min(max(share & ~31u, 32u), 256u);
 }
 
 struct WaveGen
@@ -63,22 +89,44 @@ struct WaveGen
     uint32_t block_width;
 };
 
-// Warp-aggregated append: returns this lane's first index in the queue. All lanes of the warp call.
-__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, uint32_t n)
+// A warp's appends to a queue, collected in shared memory and written 128 at a time (one atomic, whole
+// lines). Every lane calls; finish() writes the rest.
+constexpr uint32_t kQueueBatch = 128;
+struct WarpQueue
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t incl = n;
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-        if (lane >= d) incl += t;
+    uint32_t* buffer;  // kQueueBatch + 32 words of this warp
+    uint32_t* counter;
+    uint32_t* queue;
+    uint32_t held = 0;
+    __device__ __forceinline__ void write(uint32_t n)
+    {
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(counter, n);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        __syncwarp();
+        for (uint32_t j = lane; j < n; j += 32) queue[base + j] = buffer[j];
     }
-    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    uint32_t base = 0;
-    if (lane == 0 && total) base = atomicAdd(counter, total);
-    base = __shfl_sync(0xFFFFFFFFu, base, 0);
-    return base + incl - n;
-}
+    __device__ __forceinline__ void push(bool has, uint32_t value)
+    {
+        const uint32_t who = __ballot_sync(0xFFFFFFFFu, has);
+        if (has) buffer[held + (uint32_t)__popc(who & lanemask_lt())] = value;
+        held += (uint32_t)__popc(who);
+        if (held < kQueueBatch) return;
+        write(kQueueBatch);
+        held -= kQueueBatch;
+        const uint32_t rest = buffer[kQueueBatch + (threadIdx.x & 31u)];
+        __syncwarp();
+        if ((threadIdx.x & 31u) < held) buffer[threadIdx.x & 31u] = rest;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void finish()
+    {
+        if (held) write(held);
+        held = 0;
+    }
+};
+constexpr uint32_t kQueueWords = kQueueBatch + 32;
 
 // The entry (of the first `entries` of a wave) that holds item `item`, and the item within it.
 __device__ __forceinline__ uint32_t wave_entry(const WaveGen& g, uint32_t entries, uint32_t item, uint32_t& local)
@@ -99,8 +147,11 @@ __global__ void __launch_bounds__(kWaveThreads)
 {
     const uint32_t i = blockIdx.x * kWaveThreads + threadIdx.x;
     const uint32_t bw = g.block_width, bh = 32u / bw;
-    bool valid = false;
+    // Every item has its place in the first queues, those outside the image a hole: no counting (two
+    // atomics per warp on the queue lengths took four fifths of this kernel over 8 M paths).
+    if (i == 0) *counter_of(b, 0) = *counter_of(b, 1) = g.count;
     if (i < g.count) {
+        bool valid = false;
         const uint32_t item = g.first_item + i;
         uint32_t local;
         const uint32_t vs = __ldg(g.table + wave_entry(g, g.entries, item, local));
@@ -129,12 +180,8 @@ __global__ void __launch_bounds__(kWaveThreads)
             b.org[0][i] = make_float4(P.position[0], P.position[1], P.position[2], 0.0f);
             b.dir[0][i] = make_float4(d[0], d[1], d[2], 0.0f);
         }
-    }
-    const uint32_t q = warp_append(&b.counts[1], valid ? 1u : 0u);
-    const uint32_t r = warp_append(&b.counts[0], valid ? 1u : 0u);
-    if (valid) {
-        b.pathq[0][q] = i;
-        b.rayq[0][r] = i | (kKindPrimary << 30);
+        b.pathq[0][i] = valid ? i : kNone;
+        b.rayq[0][i] = valid ? i | (kKindPrimary << 30) : kNone;
     }
 }
 
@@ -183,22 +230,59 @@ __global__ void __launch_bounds__(kWaveThreads)
 __device__ __forceinline__ void begin_stage(const WaveBuffers& b, uint32_t parity)
 {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    b.counts[2 * (parity ^ 1u)] = 0;
-    b.counts[2 * (parity ^ 1u) + 1] = 0;
-    b.counts[kFetchTrace + (parity ^ 1u)] = 0;  // the next trace launch's fetch counter
-    b.counts[kCountNee] = 0;                    // this stage's light work
-    b.counts[kCountLamp] = 0;
-    b.counts[kFetchLight] = 0;
+    for (const uint32_t k : {2 * (parity ^ 1u), 2 * (parity ^ 1u) + 1, kFetchTrace + (parity ^ 1u),  // the next stage's
+                             kCountNee, kCountLamp, kFetchLight})                                     // this one's light work
+        *counter_of(b, k) = 0;
 }
 
-// Ray `i` of the queue (i < n; else none): its queue entry, view, origin, direction and length. Counts
-// the warp's rays, one atomic per (view, kind) group. Every lane calls.
-__device__ __forceinline__ bool next_ray(const WaveView* __restrict__ views, const WaveBuffers& b, uint32_t parity, bool take,
-                                         uint32_t i, uint32_t& entry, uint32_t& view, float o[3], float d[3], float& t_max)
+// The rays of a launch. With one view a lane counts its own, and the warp adds them at its end (a launch
+// traces either camera rays only or none); with several, one atomic per (view, kind) group of the warp
+// at every call (lanes whose rays change views all the time: 6.8 against 5.2 ms on 12 views when each
+// lane added its own).
+struct RayCounter
 {
-    uint32_t key = 0xFFFFFFFFu;
-    if (take) {
-        entry = b.rayq[parity][i];
+    bool one_view;
+    uint32_t paths = 0, shadows = 0;  // camera or bounce rays; shadow rays
+    bool camera = false;
+    // Every lane calls; `counted`: it has a ray of `view`.
+    __device__ __forceinline__ void add(const WaveView* __restrict__ views, bool counted, uint32_t view, uint32_t kind)
+    {
+        if (one_view) {
+            if (counted && kind == kKindShadow) ++shadows;
+            if (counted && kind != kKindShadow) ++paths;
+            camera = camera || (counted && kind == kKindPrimary);
+            return;
+        }
+        const uint32_t key = counted ? view * 4u + kind : 0xFFFFFFFFu;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
+        if (counted && (threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1u) {
+            unsigned long long* c = views[view].ray_counts;
+            if (c) atomicAdd(c + kind, (unsigned long long)__popc(peers));
+        }
+    }
+    // Every lane calls.
+    __device__ __forceinline__ void finish(const WaveView* __restrict__ views)
+    {
+        if (!one_view) return;
+        const bool cam = __any_sync(0xFFFFFFFFu, camera);
+        const uint32_t p = __reduce_add_sync(0xFFFFFFFFu, paths), s = __reduce_add_sync(0xFFFFFFFFu, shadows);
+        unsigned long long* c = views[0].ray_counts;
+        if ((threadIdx.x & 31u) != 0 || !c) return;
+        if (p) atomicAdd(c + (cam ? kKindPrimary : kKindBounce), (unsigned long long)p);
+        if (s) atomicAdd(c + kKindShadow, (unsigned long long)s);
+    }
+};
+
+// Ray `i` of the queue (`take`; else none): false for none and for a hole, else its queue entry, view,
+// origin, direction and length. Every lane calls.
+__device__ __forceinline__ bool next_ray(const WaveView* __restrict__ views, const WaveBuffers& b, uint32_t parity, bool take,
+                                         uint32_t i, uint32_t& entry, uint32_t& view, float o[3], float d[3], float& t_max,
+                                         RayCounter& counter)
+{
+    const uint32_t e = take ? b.rayq[parity][i] : kNone;
+    const bool ray = e != kNone;
+    if (ray) {
+        entry = e;
         const uint32_t slot = entry & kSlotMask, kind = entry >> 30;
         view = b.vs[slot] & 0xFFFFu;
         const float4 o4 = b.org[parity][slot];
@@ -210,14 +294,9 @@ __device__ __forceinline__ bool next_ray(const WaveView* __restrict__ views, con
         d[1] = d4.y;
         d[2] = d4.z;
         t_max = kind == kKindShadow ? d4.w : (kind == kKindPrimary ? kRayTMax : kBounceTMax);
-        key = view * 4u + kind;
     }
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-    if (take && (threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1u) {
-        unsigned long long* counts = views[view].ray_counts;
-        if (counts) atomicAdd(counts + (key & 3u), (unsigned long long)__popc(peers));
-    }
-    return take;
+    counter.add(views, ray, view, e >> 30);
+    return ray;
 }
 
 __device__ __forceinline__ void write_result(const WaveBuffers& b, uint32_t entry, const Hit& h)
@@ -228,33 +307,39 @@ __device__ __forceinline__ void write_result(const WaveBuffers& b, uint32_t entr
 }
 
 // The rays of a stage, one per lane from start to end. kEntities: the views' scenes have entities
-// (traversed after the world's bricks); the variant without them keeps the world-only DDA's registers,
-// and a fixed stride over the queue (its waves are small enough for few rays per lane).
+// (traversed after the world's bricks); the variant without them keeps the world-only DDA's registers.
+// Warps take chunks of the queue where the scene has entities or there are more than two rays per lane,
+// else a fixed stride.
 template <bool kEntities>
 __global__ void __launch_bounds__(kWaveThreads)
-    wave_trace_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity)
+    wave_trace_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, bool one_view)
 {
     grid_wait();
-    const uint32_t n = *(volatile uint32_t*)&b.counts[2 * parity];
+    const uint32_t n = count_of(b, 2 * parity);
     begin_stage(b, parity);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t stride = gridDim.x * kWaveThreads;
-    uint32_t* const fetch = &b.counts[kFetchTrace + parity];
-    for (uint32_t base = kEntities ? fetch_chunk(fetch) : blockIdx.x * kWaveThreads + (threadIdx.x & ~31u); base < n;
-         base = kEntities ? fetch_chunk(fetch) : base + stride) {
-        const uint32_t i = base + lane;
+    uint32_t* const fetch = counter_of(b, kFetchTrace + parity);
+    RayCounter counter{one_view};
+    const bool dynamic = kEntities || n > 2u * stride;
+    WarpRange range = {dynamic ? 0u : blockIdx.x * kWaveThreads + (threadIdx.x & ~31u), 0};
+    const uint32_t chunk = chunk_for(n);
+    while (dynamic ? range.more(fetch, n, chunk) : range.at < n) {
+        const uint32_t i = range.at + lane;
         uint32_t entry = 0, view = 0;
         float o[3], d[3], t_max;
-        if (next_ray(views, b, parity, i < n, i, entry, view, o, d, t_max)) {
+        if (next_ray(views, b, parity, i < n, i, entry, view, o, d, t_max, counter)) {
             Hit h;
             if constexpr (kEntities) h = trace_scene_body(views[view].scene, o, d, 0.0f, t_max, entry >> 30 == kKindShadow);
             else h = trace_ray_body(views[view].scene, o, d, 0.0f, t_max);
             write_result(b, entry, h);
         }
+        range.at += dynamic ? 32u : stride;
     }
+    counter.finish(views);
 }
 
-// The rays of a large wave (world bricks only). Rays differ widely in length: with a ray per lane from
+// The rays after the camera's of a large wave (world bricks only). They differ widely in length: with a ray per lane from
 // start to end 4 of 32 lanes were active on average on a 300 k-brick world. Here a lane that has
 // finished waits until kRefill lanes have; these write their results and take the next rays of the
 // queue together. A lane walks at most kWalkCells empty cells before the lanes that have reached a
@@ -264,18 +349,22 @@ __global__ void __launch_bounds__(kWaveThreads)
 // per lane). kRefill of 6 and 20: 12.3 and 12.4 ms on the first; kWalkCells of 3, 8, 64: 12.4, 12.2, 12.8 there
 // and 2.06, 1.97, 1.94 on the adjoint of a world without empty bricks. A pool of 64 rays per warp in
 // shared memory, taken up in phases of one kind (10 lanes, but the rays' state through shared memory
-// in every phase): 11.8, 0.84, 5.13 and 0.547 ms. Eight CTAs per SM instead of six: 12.3 ms.
+// in every phase): 11.8, 0.84, 5.13 and 0.547 ms. Eight CTAs per SM instead of six: 12.3 ms. Camera rays, whose
+// neighbours walk alike, are faster with a ray per lane (1.18 against 1.56 ms for 8.3 M).
 constexpr uint32_t kRefill = 12;
 constexpr uint32_t kWalkCells = 8;
 constexpr uint32_t kRefillPaths = 1u << 17;  // waves of more paths than this are traced so
 
 __global__ void __launch_bounds__(kWaveThreads, 6)
-    wave_trace_refill_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity)
+    wave_trace_refill_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, bool one_view)
 {
     grid_wait();
-    const uint32_t n = *(volatile uint32_t*)&b.counts[2 * parity];
+    const uint32_t n = count_of(b, 2 * parity);
     begin_stage(b, parity);
-    uint32_t* const fetch = &b.counts[kFetchTrace + parity];
+    uint32_t* const fetch = counter_of(b, kFetchTrace + parity);
+    RayCounter counter{one_view};
+    WarpRange range = {0, 0};
+    const uint32_t chunk = chunk_for(n);
     bool busy = false, done = false, left = true;  // left (warp-uniform): the queue may hold more rays
     uint32_t entry = 0, rec = 0, attrib = 0;       // of a finished ray: attrib 0 is a miss
     float t = 0.0f;
@@ -291,16 +380,17 @@ __global__ void __launch_bounds__(kWaveThreads, 6)
                 write_result(b, entry, h);
                 done = false;
             }
-            if (!left) break;
-            const uint32_t leader = (uint32_t)__ffs(free) - 1u, want = (uint32_t)__popc(free);
-            uint32_t base = 0;
-            if ((threadIdx.x & 31u) == leader) base = atomicAdd(fetch, want);
-            base = __shfl_sync(0xFFFFFFFFu, base, leader);
-            left = base + want < n;
-            const uint32_t i = base + (uint32_t)__popc(free & lanemask_lt());
+            if (left) left = range.more(fetch, n, chunk);
+            if (!left) {
+                if (free == 0xFFFFFFFFu) break;
+                continue;
+            }
+            const uint32_t i = range.at + (uint32_t)__popc(free & lanemask_lt());
+            const bool take = !busy && i < range.end;
+            range.at = min(range.at + (uint32_t)__popc(free), range.end);
             uint32_t view = 0;
             float o[3], d[3], t_max;
-            if (next_ray(views, b, parity, !busy && i < n, i, entry, view, o, d, t_max)) {
+            if (next_ray(views, b, parity, take, i, entry, view, o, d, t_max, counter)) {
                 s = &views[view].scene;
                 busy = walk_begin(*s, o, d, 0.0f, t_max, w);
                 done = !busy;
@@ -329,6 +419,7 @@ __global__ void __launch_bounds__(kWaveThreads, 6)
             done = !busy;
         }
     }
+    counter.finish(views);
 }
 
 // kMode: kShadeRender (the render), kShadeRecord (the adjoint's recording pass: also every
@@ -468,22 +559,29 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
         for (uint32_t i = threadIdx.x; i < kAlbedoCache; i += kWaveThreads) s_tag[i] = kNone;
         __syncthreads();
     }
-    const uint32_t n = *(volatile uint32_t*)&b.counts[2 * parity + 1];
+    const uint32_t n = count_of(b, 2 * parity + 1);
     const uint32_t out = parity ^ 1u;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t stride = gridDim.x * kWaveThreads;
-    if (blockIdx.x == 0 && threadIdx.x == 0) b.counts[kFetchShade + out] = 0;  // the next shade launch's
+    if (blockIdx.x == 0 && threadIdx.x == 0) *counter_of(b, kFetchShade + out) = 0;  // the next shade launch's
     // Chunks from a fetch counter (as in wave_trace_kernel) for scenes with entities or records that
     // do not stay in L2 (the 8-CTA variants); the fixed stride for the resident scene.
     constexpr bool kDynamic = kEntities || kMinBlocks == 8;
-    uint32_t* const fetch = &b.counts[kFetchShade + parity];
-    for (uint32_t base = kDynamic ? fetch_chunk(fetch) : blockIdx.x * kWaveThreads + (threadIdx.x & ~31u); base < n;
-         base = kDynamic ? fetch_chunk(fetch) : base + stride) {
-        const uint32_t i = base + lane;
+    uint32_t* const fetch = counter_of(b, kFetchShade + parity);
+    __shared__ uint32_t s_queue[kWaveThreads / 32][4][kQueueWords];
+    uint32_t(*const buffers)[kQueueWords] = s_queue[threadIdx.x >> 5];
+    WarpQueue paths = {buffers[0], counter_of(b, 2 * out + 1), b.pathq[out]};
+    WarpQueue rays = {buffers[1], counter_of(b, 2 * out), b.rayq[out]};
+    WarpQueue draws = {buffers[2], counter_of(b, kCountNee), b.neeq};
+    WarpQueue lamps = {buffers[3], counter_of(b, kCountLamp), b.lampq};
+    WarpRange range = {kDynamic ? 0u : blockIdx.x * kWaveThreads + (threadIdx.x & ~31u), 0};
+    const uint32_t chunk = chunk_for(n);
+    for (; kDynamic ? range.more(fetch, n, chunk) : range.at < n; range.at += kDynamic ? 32u : stride) {
+        const uint32_t i = range.at + lane;
         uint32_t slot = 0;
         bool live = false, nee = false, lamp = false, ext = false;
-        if (i < n) {
-            slot = b.pathq[parity][i];
+        if (i < n) slot = b.pathq[parity][i];
+        if (i < n && slot != kNone) {
             const uint32_t f = b.flags[slot];
             const uint32_t vs = b.vs[slot];
             const WaveView& V = views[vs & 0xFFFFu];
@@ -660,15 +758,15 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
             }
             if (finish) finish_path<kMode>(V, b, adj, slot, item, sp, zero, rad, e0, a0, resolve);
         }
-        const uint32_t q = warp_append(&b.counts[2 * out + 1], live ? 1u : 0u);
-        if (live) b.pathq[out][q] = slot;
-        const uint32_t r = warp_append(&b.counts[2 * out], ext ? 1u : 0u);
-        if (ext) b.rayq[out][r] = slot | (kKindBounce << 30);
-        const uint32_t d = warp_append(&b.counts[kCountNee], nee ? 1u : 0u);
-        if (nee) b.neeq[d] = slot;
-        const uint32_t l = warp_append(&b.counts[kCountLamp], lamp ? 1u : 0u);
-        if (lamp) b.lampq[l] = slot | (live ? 0u : kLampEnds);
+        paths.push(live, slot);
+        rays.push(ext, slot | (kKindBounce << 30));
+        draws.push(nee, slot);
+        lamps.push(lamp, slot | (live ? 0u : kLampEnds));
     }
+    paths.finish();
+    rays.finish();
+    draws.finish();
+    lamps.finish();
     if (kMode == kShadeReplay) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < kAlbedoCache * 3; i += kWaveThreads) {
@@ -716,14 +814,16 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
         for (uint32_t i = threadIdx.x; i < kAlbedoCache; i += kWaveThreads) s_tag[i] = kNone;
         __syncthreads();
     }
-    const uint32_t draws = *(volatile uint32_t*)&b.counts[kCountNee];
-    const uint32_t lamps = *(volatile uint32_t*)&b.counts[kCountLamp];
+    const uint32_t draws = count_of(b, kCountNee);
+    const uint32_t lamps = count_of(b, kCountLamp);
     constexpr uint32_t chunk = kQuad ? 8u : 32u;
     const uint32_t draw_chunks = (draws + chunk - 1) / chunk;
     const uint32_t chunks = draw_chunks + (lamps + chunk - 1) / chunk;
     const uint32_t out = parity ^ 1u;
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t* const fetch = &b.counts[kFetchLight];
+    uint32_t* const fetch = counter_of(b, kFetchLight);
+    __shared__ uint32_t s_queue[kWaveThreads / 32][kQueueWords];
+    WarpQueue rays = {s_queue[threadIdx.x >> 5], counter_of(b, 2 * out), b.rayq[out]};
     for (uint32_t c = fetch_one(fetch); c < chunks; c = fetch_one(fetch)) {
         const bool draw = c < draw_chunks;
         const uint32_t base = (draw ? c : c - draw_chunks) * chunk;
@@ -811,8 +911,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
                     }
                 }
             }
-            const uint32_t q = warp_append(&b.counts[2 * out], shadow ? 1u : 0u);
-            if (shadow) b.rayq[out][q] = slot | (kKindShadow << 30);
+            rays.push(shadow, slot | (kKindShadow << 30));
         } else {
             Hit h;
             LampHit lamp = {nullptr, 0u, kNone, 0.0f};
@@ -888,6 +987,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
             }
         }
     }
+    rays.finish();
     if (kMode == kShadeReplay) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < kAlbedoCache * 3; i += kWaveThreads) {
@@ -965,6 +1065,7 @@ uint32_t WavePlan::largest() const
 WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_width, uint32_t slots)
 {
     WavePlan plan;
+    plan.one_view = view_count == 1;
     uint32_t max_spp = 0;
     for (uint32_t v = 0; v < view_count; ++v) max_spp = std::max(max_spp, views[v].params.spp);
     const uint32_t bh = 32u / block_width;
@@ -1067,14 +1168,16 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
             // At most a light draw and a lamp hit per path; chunks of 32.
             const uint32_t light_grid = std::min<uint32_t>((2 * n + kWaveThreads - 1) / kWaveThreads,
                                                            sm_count * (uint32_t)light_blocks[entities ? 1 : 0]);
+            const bool one_view = plan.one_view;
             const bool quad = n <= kQuadPaths;
             const bool refill = !entities && n > kRefillPaths;
             const uint32_t refill_grid = sm_count * (uint32_t)refill_blocks;
             const uint32_t quad_grid = std::min<uint32_t>((8 * n + kWaveThreads - 1) / kWaveThreads, sm_count * 5);
-            const auto stage = [&](auto with_entities, uint32_t parity) {
+            const auto stage = [&](auto with_entities, uint32_t it) {
+                const uint32_t parity = it & 1u;
                 constexpr bool kEntities = decltype(with_entities)::value;
-                cudaError_t e = refill ? launch(wave_trace_refill_kernel, refill_grid, stream, d_views, b, parity)
-                                     : launch(wave_trace_kernel<kEntities>, ray_grid, stream, d_views, b, parity);
+                cudaError_t e = refill && it > 0 ? launch(wave_trace_refill_kernel, refill_grid, stream, d_views, b, parity, one_view)
+                                     : launch(wave_trace_kernel<kEntities>, ray_grid, stream, d_views, b, parity, one_view);
                 if (e == cudaSuccess)
                     e = launch(wave_shade_kernel<kMode, kMinBlocks, kEntities>, shade_grid, stream, d_views, b, parity, adj,
                                resolve);
@@ -1086,7 +1189,7 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
                 return e;
             };
             for (uint32_t it = 0; it <= plan.bounces[s]; ++it) {
-                CX_TRY(entities ? stage(std::true_type{}, it & 1u) : stage(std::false_type{}, it & 1u));
+                CX_TRY(entities ? stage(std::true_type{}, it) : stage(std::false_type{}, it));
                 count += 3;
             }
             if (resolve && kMode != kShadeReplay) {
