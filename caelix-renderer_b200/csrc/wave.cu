@@ -299,6 +299,17 @@ __device__ __forceinline__ bool next_ray(const WaveView* __restrict__ views, con
     return ray;
 }
 
+// The rays that a warp takes at a time: 32, or where the queue fills less than three eighths of the grid's
+// lanes 8 or 4 of them in more warps. The lanes of a warp run one after another where their rays differ,
+// and these launches last as long as their longest warp. Measured (one B200, 1 spp): 80 x 60 0.182 -> 0.155
+// ms, 160 x 90 0.119 -> 0.105, 200 x 150 0.241 -> 0.218, 256 x 200 on 5 k bricks 0.305 -> 0.286, 256 x 256 on 20 k
+// 0.382 -> 0.371. With 16 rays from half of the lanes down and 8 from a quarter (in the refilling kernel
+// too): 512 x 512 0.424 -> 0.536, the lanes no longer neighbours.
+__device__ __forceinline__ uint32_t rays_per_warp(uint32_t n, uint32_t warps)
+{
+    return n > 12u * warps ? 32u : (n > 4u * warps ? 8u : 4u);
+}
+
 __device__ __forceinline__ void write_result(const WaveBuffers& b, uint32_t entry, const Hit& h)
 {
     const uint32_t slot = entry & kSlotMask;
@@ -308,8 +319,8 @@ __device__ __forceinline__ void write_result(const WaveBuffers& b, uint32_t entr
 
 // The rays of a stage, one per lane from start to end. kEntities: the views' scenes have entities
 // (traversed after the world's bricks); the variant without them keeps the world-only DDA's registers.
-// Warps take chunks of the queue where the scene has entities or there are more than two rays per lane,
-// else a fixed stride.
+// Warps take chunks of the queue where there are more than two rays per lane (with entities, whose rays
+// differ more, from one on), else a fixed stride.
 template <bool kEntities>
 __global__ void __launch_bounds__(kWaveThreads)
     wave_trace_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, bool one_view)
@@ -318,14 +329,15 @@ __global__ void __launch_bounds__(kWaveThreads)
     const uint32_t n = count_of(b, 2 * parity);
     begin_stage(b, parity);
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t stride = gridDim.x * kWaveThreads;
+    const uint32_t warps = gridDim.x * (kWaveThreads / 32);
+    const uint32_t lanes = rays_per_warp(n, warps);
     uint32_t* const fetch = counter_of(b, kFetchTrace + parity);
     RayCounter counter{one_view};
-    const bool dynamic = kEntities || n > 2u * stride;
-    WarpRange range = {dynamic ? 0u : blockIdx.x * kWaveThreads + (threadIdx.x & ~31u), 0};
+    const bool dynamic = n > 64u * warps || (kEntities && lanes == 32u);
+    WarpRange range = {dynamic ? 0u : (blockIdx.x * (kWaveThreads / 32) + threadIdx.x / 32) * lanes, 0};
     const uint32_t chunk = chunk_for(n);
     while (dynamic ? range.more(fetch, n, chunk) : range.at < n) {
-        const uint32_t i = range.at + lane;
+        const uint32_t i = lane < lanes ? range.at + lane : n;
         uint32_t entry = 0, view = 0;
         float o[3], d[3], t_max;
         if (next_ray(views, b, parity, i < n, i, entry, view, o, d, t_max, counter)) {
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(kWaveThreads)
             else h = trace_ray_body(views[view].scene, o, d, 0.0f, t_max);
             write_result(b, entry, h);
         }
-        range.at += dynamic ? 32u : stride;
+        range.at += dynamic ? 32u : warps * lanes;
     }
     counter.finish(views);
 }
@@ -1161,7 +1173,8 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
             CX_TRY(cudaMemsetAsync(b.counts, 0, 4 * kCountWords, stream));
             wave_generate_kernel<<<(n + kWaveThreads - 1) / kWaveThreads, kWaveThreads, 0, stream>>>(d_views, g, b);
             ++count;
-            const uint32_t ray_grid = std::min<uint32_t>((2 * n + kWaveThreads - 1) / kWaveThreads,
+            // (At least four rays per warp.)
+            const uint32_t ray_grid = std::min<uint32_t>((2 * n + kWaveThreads / 8 - 1) / (kWaveThreads / 8),
                                                          sm_count * (uint32_t)trace_blocks[entities ? 1 : 0]);
             const uint32_t shade_grid = std::min<uint32_t>((n + kWaveThreads - 1) / kWaveThreads,
                                                            sm_count * (uint32_t)shade_blocks[entities ? 1 : 0]);
