@@ -1,5 +1,5 @@
 // The scene build (scene.cuh): brick records (finalize), the canonical brick hash table, the
-// brick occupancy bitmap, the light records in group light blocks, and the light tree.
+// cell table (occupancy and first record per 32 brick cells), the light records in group light blocks, and the light tree.
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -1,4 +1,5 @@
-// Device functions of the brick hash table shared by the scene build and the trace kernels.
+// Device functions of the brick tables: the hash functions of the canonical hash table (the scene
+// build) and the lookups in the cell table (the build and the trace kernels).
 //
 // The key slot layout and the fingerprint are the reference's hash module
 // (lib/src/rhi/hash_table_layout.h:24-34: 16-byte slots key_lo, key_hi, payload, pad;
@@ -34,21 +35,6 @@ __host__ __device__ __forceinline__ void hash_fingerprint(int32_t x, int32_t y, 
 __host__ __device__ __forceinline__ uint32_t hash_home(uint32_t key_lo, uint32_t capacity)
 {
     return (uint32_t)(((uint64_t)key_lo * capacity) >> 32);
-}
-
-// The record of brick (x, y, z), or 0xFFFFFFFF.
-__device__ __forceinline__ uint32_t hash_lookup(const uint4* __restrict__ slots, uint32_t capacity, uint32_t max_probe,
-                                                int32_t x, int32_t y, int32_t z)
-{
-    uint32_t lo, hi;
-    hash_fingerprint(x, y, z, lo, hi);
-    const uint32_t home = hash_home(lo, capacity);
-    for (uint32_t p = home; p <= home + max_probe; ++p) {
-        const uint4 s = __ldg(slots + p);
-        if (s.x == 0u) return 0xFFFFFFFFu;
-        if (s.x == lo && s.y == hi) return s.z;
-    }
-    return 0xFFFFFFFFu;
 }
 
 // The brick of linear brick index `lin` in the cell table: the records are in

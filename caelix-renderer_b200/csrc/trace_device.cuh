@@ -1,10 +1,10 @@
 // Device functions of the path tracer, shared by the per-frame kernel (trace.cu) and the batched
-// persistent kernel (trace_batch.cu); each translation unit compiles its own copy. Restates, as
+// persistent kernel (trace_batch.cu) and the wavefront kernels (wave.cu); each translation unit compiles its own copy. Restates, as
 // device code:
 //   brick DDA          shaders/render/caelix_brick_trace.hlsl:177-451
 //   scene traversal    shaders/render/caelix_scene_trace.hlsl:57-169, the TLAS replaced by a
-//                      front-to-back DDA over the brick grid: the occupancy bitmap, then the brick
-//                      hash table, then the brick DDA; the first brick in DDA order with a hit in
+//                      front-to-back DDA over the brick grid: the cell table (occupancy and record of
+//                      a brick cell in one 8-byte load), then the brick DDA; the first brick in DDA order with a hit in
 //                      [tmin, tmax) is the closest hit
 //   light tree draw    shaders/light/caelix_light_tree.hlsl:65-767
 //   light tree pdf     caelix_light_tree.hlsl:514-608, 769-777, 853-949

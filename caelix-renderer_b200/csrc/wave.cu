@@ -17,6 +17,7 @@
 // bit. Queues are compacted with warp-aggregated atomics; every kernel reads its queue length on
 // the device, so a whole frame is recorded without a host synchronisation (graph-capturable).
 #include <algorithm>
+#include <mutex>
 #include <cstdint>
 #include <type_traits>
 
@@ -1135,7 +1136,11 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
 {
     if (b.capacity == 0) return cudaErrorInvalidValue;
     static int trace_blocks[2] = {0, 0}, refill_blocks = 0, shade_blocks[2] = {0, 0}, light_blocks[2] = {0, 0};
-    if (trace_blocks[0] == 0) {
+    // Asked once; the lock keeps a second thread from reading a half-filled set.
+    static std::mutex blocks_mutex;
+    static bool blocks_known = false;
+    std::unique_lock<std::mutex> blocks_lock(blocks_mutex);
+    if (!blocks_known) {
         CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&trace_blocks[0], wave_trace_kernel<false>,
                                                              kWaveThreads, 0));
         CX_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&trace_blocks[1], wave_trace_kernel<true>, kWaveThreads,
@@ -1155,7 +1160,9 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
             trace_blocks[k] = std::max(trace_blocks[k], 1);
             shade_blocks[k] = std::max(shade_blocks[k], 1);
         }
+        blocks_known = true;
     }
+    blocks_lock.unlock();
     uint32_t count = 0;
     for (size_t s = 0; s < plan.items.size(); ++s) {
         // Several sample indices: the whole wave in one sub-wave, then the samples' sums.
