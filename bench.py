@@ -57,14 +57,14 @@ SORT_STAGE_BYTES_PER_PAIR = 60.0
 # The build's dominant stage: the tile kernel and the upper aggregation (aggregation 52 B read +
 # 48 B written, 4-wide collapse 96 x 1/2 read + 224 x 1/2 written, per leaf).
 TILE_STAGE_BYTES_PER_LEAF = 100.0 + 160.0
-TRACE_BYTES_PER_RAY = 64  # lower bound: one hash slot sector + one record sector per ray
+TRACE_BYTES_PER_RAY = 64  # lower bound: one cell-table sector + one record sector per ray
 # DRAM bytes (read + write) measured by ncu (one capture per kernel, cold cache; profiles/): the sort
 # stage at 4,194,304 pairs (a pipelined pass times four), scaled per pair; the tile stage at
 # 2,097,152 leaves (lt_tile_kernel + lt_aggregate_upper_kernel), scaled per leaf; the wavefront
-# frame of the 512 x 512 trace (trace and shade kernels of its 5 bounce iterations).
+# frame of the 512 x 512 trace (trace, shade and light kernels of its 5 bounce iterations).
 SORT_STAGE_DRAM_BYTES_PER_PAIR = 4 * 34.2e6 / 4194304
 TILE_STAGE_DRAM_BYTES_PER_LEAF = (236.7e6 + 378.4e6 + 25.4e6 + 3.1e6) / 2097152
-TRACE_FRAME_DRAM_BYTES = 134.7e6
+TRACE_FRAME_DRAM_BYTES = 180.5e6
 
 
 def measured_peaks():
@@ -576,7 +576,7 @@ def measure_trace(args, world, local, dev, stream, flush):
         "value": value,
         "ms_per_step": ms,
         "rays_per_step": rays_per_step,
-        "roofline": {"kernel": "wave_trace_kernel + wave_shade_kernel (the frame)", "bound": "hbm",
+        "roofline": {"kernel": "wave_trace(_refill), wave_shade and wave_light kernels (the frame)", "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": TRACE_FRAME_DRAM_BYTES,
                      "traffic_source": "ncu launch list: DRAM bytes of one frame's wave kernels (cold cache)",
@@ -744,7 +744,7 @@ def measure_large(args, world, local, dev, stream, flush, rank):
     }
     peak, peak_kind = measured_peaks()
     achieved = TRACE_BYTES_PER_RAY * (rays / steps) / (ms / 1e3) / 1e9
-    result["roofline"] = {"kernel": "wave_trace_kernel + wave_shade_kernel (the frame)", "bound": "hbm",
+    result["roofline"] = {"kernel": "wave_trace(_refill), wave_shade and wave_light kernels (the frame)", "bound": "hbm",
                           "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                           "peak_kind": peak_kind, "traffic": None, "bytes_per_ray": TRACE_BYTES_PER_RAY,
                           "note": "latency-bound ray traversal; the bytes are a per-ray lower bound"}

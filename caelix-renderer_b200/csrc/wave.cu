@@ -551,10 +551,10 @@ __device__ __forceinline__ void replay_vertex(const SceneView& S, const WaveAdjo
         if (al[k] > 0.0f && G[k] != 0.0f) cache.add(code, k, G[k] * (R[k] - rad[k]) / al[k]);
 }
 
-// kMinBlocks CTAs of 128 threads per SM: 5 (96 registers, few spills) for a scene whose records
-// stay in L2, 8 (64 registers) where the descent and the record loads go to HBM and more warps
-// in flight hide them (measured: 5 is the fastest of 3 .. 8 on the 128^3 world; 8 on the
-// 2 M-brick world and the 64-scene batch).
+// kMinBlocks CTAs of 128 threads per SM: 5 (96 registers, no spills) for a scene whose records
+// stay in L2, 8 (64 registers; the light kernels spill about 150 bytes) where the descent and the
+// record loads go to HBM and more warps in flight hide them (measured: 5 is the fastest of 3 .. 8 on
+// the 128^3 world; 8 on the 2 M-brick world and the 64-scene batch).
 // kEntities: the views' scenes have entities (their hits, their lights); the variant without
 // them keeps the world-only shading's registers. resolve: a finished path leaves its sample in its
 // slot for wave_resolve_kernel (several samples of a pixel are in flight).
