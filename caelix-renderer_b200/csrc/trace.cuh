@@ -71,7 +71,7 @@ struct WaveBuffers
 {
     uint32_t capacity = 0;  // slots
     uint32_t* item = nullptr;   // pixel index within the view (y * width + x)
-    uint32_t* vs = nullptr;     // view | sample << 16
+    uint32_t* vs = nullptr;     // view | sample of the wave << 16
     uint32_t* flags = nullptr;
     uint32_t* rng = nullptr;
     uint32_t* light_rng = nullptr;
@@ -128,7 +128,8 @@ WaveBuffers wave_carve(void* base, uint32_t capacity);
 // then runs one sample at a time). At 2^23 slots the path state is 2.1 GB, of 180.
 struct WavePlan
 {
-    std::vector<uint32_t> table;     // per wave: entries (view | sample << 16), then item bases
+    std::vector<uint32_t> table;     // per wave: entries (view | sample of the wave << 16), then item bases
+    std::vector<uint32_t> first;     // per wave: its first sample index
     std::vector<uint32_t> offset;    // per wave: first word of its entries in `table`
     std::vector<uint32_t> entries;   // per wave: number of entries
     std::vector<uint32_t> samples;   // per wave: sample indices
@@ -138,6 +139,7 @@ struct WavePlan
     uint32_t largest() const;        // the items of the largest wave
 };
 constexpr uint32_t kWaveMergeSlots = 1u << 23;
+constexpr uint32_t kWaveMaxSamples = 1u << 16;  // of a wave: an entry's sample has 16 bits
 WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_width, uint32_t slots);
 // The plan's `slots` for a single view's render or adjoint with a wave capacity (0: not set).
 inline uint32_t wave_merge_slots(uint32_t wave_capacity)

@@ -82,9 +82,10 @@ __device__ __forceinline__ uint32_t chunk_for(uint32_t n)
 
 struct WaveGen
 {
-    const uint32_t* table;  // entries (view | sample << 16), then item bases (`entries` each)
+    const uint32_t* table;  // entries (view | sample << 16, of the wave), then item bases (`entries` each)
     uint32_t entries;
-    uint32_t samples;  // sample indices of the wave
+    uint32_t first_sample;  // the entries' samples count from it
+    uint32_t samples;       // sample indices of the wave
     uint32_t first_item;
     uint32_t count;
     uint32_t block_width;
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kWaveThreads)
     const uint32_t px = (blk % V.blocks_x) * bw + in % bw;
     const uint32_t py = (blk / V.blocks_x) * bh + in / bw;
     if (px >= P.width || py >= P.height) return;
-    const uint32_t first = vs >> 16;
+    const uint32_t first = g.first_sample;
     float* o = V.radiance + 3ull * (py * P.width + px);
     float acc[3] = {0.0f, 0.0f, 0.0f};
     if (first != 0) {
@@ -561,7 +562,7 @@ __device__ __forceinline__ void replay_vertex(const SceneView& S, const WaveAdjo
 template <int kMode, int kMinBlocks, bool kEntities>
 __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     wave_shade_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj,
-                      bool resolve)
+                      bool resolve, uint32_t first_sample)
 {
     grid_wait();
     __shared__ float s_albedo[kMode == kShadeReplay ? kAlbedoCache * 3 : 1];
@@ -600,7 +601,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
             const WaveView& V = views[vs & 0xFFFFu];
             const SceneView& S = V.scene;
             const TraceParams& P = V.params;
-            const uint32_t sp = vs >> 16;
+            const uint32_t sp = first_sample + (vs >> 16);
             const uint32_t item = b.item[slot];
             const bool primary = (f & kFlagPrimary) != 0;
             float rad[3] = {0.0f, 0.0f, 0.0f};
@@ -816,7 +817,7 @@ __device__ __forceinline__ uint32_t fetch_one(uint32_t* counter)
 template <int kMode, int kMinBlocks, bool kEntities, bool kQuad>
 __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
     wave_light_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, const WaveAdjoint adj,
-                      bool resolve)
+                      bool resolve, uint32_t first_sample)
 {
     grid_wait();
     __shared__ float s_albedo[kMode == kShadeReplay ? kAlbedoCache * 3 : 1];
@@ -993,7 +994,7 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
                     const float4 e4 = b.e0[slot];
                     const float a0[3] = {a4.x, a4.y, a4.z};
                     const float e0[3] = {e4.x, e4.y, e4.z};
-                    finish_path<kMode>(V, b, adj, slot, b.item[slot], vs >> 16, false, rad, e0, a0, resolve);
+                    finish_path<kMode>(V, b, adj, slot, b.item[slot], first_sample + (vs >> 16), false, rad, e0, a0, resolve);
                 } else {
                     b.radiance[slot] = make_float4(rad[0], rad[1], rad[2], 0.0f);
                 }
@@ -1097,14 +1098,16 @@ WavePlan wave_plan(const WaveView* views, uint32_t view_count, uint32_t block_wi
             bounces = std::max(bounces, p.bounce_count);
             left = std::min(left, p.spp - s);
         }
-        const uint32_t samples = items ? (uint32_t)std::min<uint64_t>(left, std::max<uint64_t>(slots / items, 1)) : 1u;
+        uint32_t samples = items ? (uint32_t)std::min<uint64_t>(left, std::max<uint64_t>(slots / items, 1)) : 1u;
+        samples = std::min(samples, kWaveMaxSamples);
+        plan.first.push_back(s);
         plan.offset.push_back((uint32_t)plan.table.size());
         plan.entries.push_back((uint32_t)ids.size() * samples);
         plan.samples.push_back(samples);
         plan.items.push_back((uint32_t)std::min<uint64_t>(items * samples, 0xFFFFFFFFull));
         plan.bounces.push_back(bounces);
         for (uint32_t k = 0; k < samples; ++k)
-            for (uint32_t id : ids) plan.table.push_back(id | ((s + k) << 16));
+            for (uint32_t id : ids) plan.table.push_back(id | (k << 16));
         uint64_t base = 0;
         for (uint32_t k = 0; k < samples; ++k)
             for (uint32_t size : sizes) {
@@ -1173,6 +1176,7 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
             WaveGen g;
             g.table = d_table + plan.offset[s];
             g.entries = plan.entries[s];
+            g.first_sample = plan.first[s];
             g.samples = plan.samples[s];
             g.first_item = first;
             g.count = n;
@@ -1200,12 +1204,12 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
                                      : launch(wave_trace_kernel<kEntities>, ray_grid, stream, d_views, b, parity, one_view);
                 if (e == cudaSuccess)
                     e = launch(wave_shade_kernel<kMode, kMinBlocks, kEntities>, shade_grid, stream, d_views, b, parity, adj,
-                               resolve);
+                               resolve, g.first_sample);
                 if (e == cudaSuccess)
                     e = quad ? launch(wave_light_kernel<kMode, 5, kEntities, true>, quad_grid, stream, d_views, b, parity, adj,
-                                      resolve)
+                                      resolve, g.first_sample)
                              : launch(wave_light_kernel<kMode, kMinBlocks, kEntities, false>, light_grid, stream, d_views, b,
-                                      parity, adj, resolve);
+                                      parity, adj, resolve, g.first_sample);
                 return e;
             };
             for (uint32_t it = 0; it <= plan.bounces[s]; ++it) {
