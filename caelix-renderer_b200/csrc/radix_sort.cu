@@ -578,18 +578,18 @@ void radix_histogram(const uint32_t* keys, uint32_t n, uint32_t* hist, uint32_t 
 void onesweep_sort(uint32_t* keys_a, uint32_t* values_a, uint32_t* keys_b, uint32_t* values_b, uint32_t n,
                    bool identity_values, uint32_t* scratch, uint32_t* status, cudaStream_t stream,
                    const SortGather* gather, uint32_t keys_per_thread, const SortWaitTest* wait_test,
-                   uint32_t key_bits)
+                   uint32_t key_bits, bool after_kernel)
 {
     if (n == 0) return;
     const uint32_t passes = key_bits >= 32 ? 4u : std::max(1u, (key_bits + 7u) / 8u);
     if (n <= kSmallSortKeys) {
         const SortGather g = gather ? *gather : SortGather{nullptr, 0, nullptr, nullptr};
         if (n <= kRankSortKeys) {
-            launch_chained(identity_values ? rank_sort_kernel<true> : rank_sort_kernel<false>, 1, kSortThreads, 0, stream, keys_a,
-                           values_a, n, g);
+            launch_kernel(after_kernel, identity_values ? rank_sort_kernel<true> : rank_sort_kernel<false>, 1, kSortThreads, 0,
+                          stream, keys_a, values_a, n, g);
         } else {
-            launch_chained(identity_values ? small_sort_kernel<true> : small_sort_kernel<false>, 1, kSortThreads, 0, stream,
-                           keys_a, values_a, n, passes, g);
+            launch_kernel(after_kernel, identity_values ? small_sort_kernel<true> : small_sort_kernel<false>, 1, kSortThreads, 0,
+                          stream, keys_a, values_a, n, passes, g);
         }
         return;
     }

@@ -103,11 +103,12 @@ struct SortWaitTest
 // passes in shared memory (one launch; the same permutation; scratch and histograms unused).
 // `key_bits`: every key is below 2^key_bits, so only the passes of its low ceil(key_bits / 8) digits
 // run (an odd count of passes ends with a copy of the result back into keys_a / values_a).
-// The launches are chained (launch.cuh): the command before them in `stream` is a kernel.
+// The launches are chained (launch.cuh). `after_kernel`: the command before them in `stream` is a kernel as
+// the chain needs it (above kSmallSortKeys it always is: the histograms'); false: the first launch is plain.
 void onesweep_sort(uint32_t* keys_a, uint32_t* values_a, uint32_t* keys_b, uint32_t* values_b, uint32_t n,
                    bool identity_values, uint32_t* scratch, uint32_t* status, cudaStream_t stream,
                    const SortGather* gather = nullptr, uint32_t keys_per_thread = kSortKeysPerThread,
-                   const SortWaitTest* wait_test = nullptr, uint32_t key_bits = 32);
+                   const SortWaitTest* wait_test = nullptr, uint32_t key_bits = 32, bool after_kernel = true);
 
 // The number of bits of the values below `bound` (0 for bound <= 1).
 inline uint32_t bits_below(uint64_t bound)

@@ -90,8 +90,9 @@ CAELIX_API CaelixResult caelix_radix_sort_pairs_static(uint32_t* keys, uint32_t*
         const uint32_t grid = std::min<uint32_t>((count + 2047) / 2048, cx::current_sm_count() * 4);
         cx::radix_histogram(keys, count, scratch, grid, s);
     }
+    // Up to kSmallSortKeys pairs the sort's one kernel comes right after the caller's commands: a plain launch.
     cx::onesweep_sort(keys, values, keys_b, values_b, count, identity_values != 0, scratch,
-                      status ? status : fallback_status, s);
+                      status ? status : fallback_status, s, nullptr, cx::kSortKeysPerThread, nullptr, 32, count > cx::kSmallSortKeys);
     return cx::cuda_result(cudaGetLastError(), "caelix_radix_sort_pairs_static");
 }
 
