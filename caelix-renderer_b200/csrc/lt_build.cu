@@ -23,9 +23,9 @@ __device__ __forceinline__ float hmax(float a, float b) { return b > a ? b : a; 
 
 __device__ __forceinline__ LightSummary load_summary(const LightSummary* p)
 {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    const float4 c = __ldg(reinterpret_cast<const float4*>(p) + 2);
+    const float4 a = chain_load(reinterpret_cast<const float4*>(p));
+    const float4 b = chain_load(reinterpret_cast<const float4*>(p) + 1);
+    const float4 c = chain_load(reinterpret_cast<const float4*>(p) + 2);
     LightSummary s;
     s.face[0] = a.x; s.face[1] = a.y; s.face[2] = a.z; s.face[3] = a.w;
     s.face[4] = b.x; s.face[5] = b.y; s.lo[0] = b.z; s.lo[1] = b.w;
@@ -307,7 +307,7 @@ __device__ __forceinline__ uint32_t centre_key(const float4 ctr, const float lo[
 // Morton codes (value = leaf index) from the box centres the emit wrote + the four digit histograms
 // + clearing the arrival counters and the range-count differences.
 __global__ void __launch_bounds__(kThreads)
-    lt_morton_kernel(const float4* __restrict__ centres, uint32_t n, const BuildControl* __restrict__ control,
+    lt_morton_kernel(const float4* centres, uint32_t n, const BuildControl* control,
                      uint32_t* __restrict__ keys, uint32_t* __restrict__ counter, uint32_t* __restrict__ cover,
                      uint32_t* __restrict__ hist)
 {
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kThreads)
     for (int k = 0; k < 3; ++k) extent[k] = hmax(hi[k] - lo[k], 1e-6f);
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t key = centre_key(__ldg(centres + i), lo, extent);
+        const uint32_t key = centre_key(chain_load(centres + i), lo, extent);
         keys[i] = key;
         counter[i] = 0;
         cover[i] = 0;
@@ -402,14 +402,14 @@ __device__ __forceinline__ void store_node(const KarrasNode& o, uint32_t i, uint
 }
 
 __global__ void __launch_bounds__(kThreads)
-    lt_karras_kernel(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ left,
+    lt_karras_kernel(const uint32_t* keys, int n, uint32_t* __restrict__ left,
                      uint32_t* __restrict__ right, uint32_t* __restrict__ parent, uint32_t* __restrict__ leaf_parent,
                      uint32_t* __restrict__ cover, uint32_t* __restrict__ range_end)
 {
     grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
-    const KarrasNode o = karras_node([&](int j) { return __ldg(keys + j); }, i, n);
+    const KarrasNode o = karras_node([&](int j) { return chain_load(keys + j); }, i, n);
     store_node(o, (uint32_t)i, left, right, parent, leaf_parent, range_end);
     atomicAdd(cover + o.a, 1u);
     atomicAdd(cover + o.b, 0xFFFFFFFFu);
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kThreads)
 // two scans 12.2; the whole build 85 -> 56 us. By one CTA of 1,024 threads instead, radix passes took 27
 // us, and with Karras and the scans behind them 49; ranks whose CTAs made the keys themselves 18.5.
 __global__ void __launch_bounds__(kThreads)
-    lt_small_keys_kernel(const float4* __restrict__ centres, uint32_t n, const BuildControl* __restrict__ control,
+    lt_small_keys_kernel(const float4* centres, uint32_t n, const BuildControl* control,
                          uint32_t* __restrict__ keys, uint32_t* __restrict__ counter, uint32_t* __restrict__ cover)
 {
     grid_wait();
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kThreads)
     decode_bounds(control, lo, hi);
 #pragma unroll
     for (int k = 0; k < 3; ++k) extent[k] = hmax(hi[k] - lo[k], 1e-6f);
-    keys[i] = centre_key(__ldg(centres + i), lo, extent);
+    keys[i] = centre_key(chain_load(centres + i), lo, extent);
     counter[i] = 0;
     cover[i] = 0;
 }
@@ -445,12 +445,12 @@ constexpr uint32_t kRankLeaves = kRankThreads / 32;  // per CTA
 // The first n keys into shared memory (the arrays are carved on 256-byte boundaries: whole 16-byte
 // words may be read), the words past them filled with a value above every key.
 template <uint32_t kCta>
-__device__ __forceinline__ void copy_keys(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* s_keys, uint32_t padded)
+__device__ __forceinline__ void copy_keys(const uint32_t* keys, uint32_t n, uint32_t* s_keys, uint32_t padded)
 {
 #pragma unroll 4
     for (uint32_t j = threadIdx.x; j < padded / 4; j += kCta) {
         uint4 v = make_uint4(kNone, kNone, kNone, kNone);
-        if (4 * j < n) v = __ldg(reinterpret_cast<const uint4*>(keys) + j);
+        if (4 * j < n) v = chain_load(reinterpret_cast<const uint4*>(keys) + j);
         if (4 * j + 1 >= n) v.y = kNone;
         if (4 * j + 2 >= n) v.z = kNone;
         if (4 * j + 3 >= n) v.w = kNone;
@@ -459,7 +459,7 @@ __device__ __forceinline__ void copy_keys(const uint32_t* __restrict__ keys, uin
 }
 
 __global__ void __launch_bounds__(kRankThreads)
-    lt_rank_sort_kernel(const uint32_t* __restrict__ keys_in, uint32_t n, uint32_t* __restrict__ keys,
+    lt_rank_sort_kernel(const uint32_t* keys_in, uint32_t n, uint32_t* __restrict__ keys,
                         uint32_t* __restrict__ values)
 {
     __shared__ __align__(16) uint32_t s_keys[kSmallSortKeys];
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kRankThreads)
 constexpr uint32_t kSmallKarrasThreads = 64;
 
 __global__ void __launch_bounds__(kSmallKarrasThreads)
-    lt_small_karras_kernel(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ left,
+    lt_small_karras_kernel(const uint32_t* keys, uint32_t n, uint32_t* __restrict__ left,
                            uint32_t* __restrict__ right, uint32_t* __restrict__ parent, uint32_t* __restrict__ leaf_parent,
                            uint32_t* __restrict__ cover, uint32_t* __restrict__ range_end)
 {
@@ -512,7 +512,7 @@ constexpr int kSmallScanItems = kSmallSortKeys / kSmallScanThreads;
 static_assert(kSmallScanItems == 4, "nodes per thread");
 
 __global__ void __launch_bounds__(kSmallScanThreads)
-    lt_small_scan_kernel(uint32_t nodes, const uint32_t* __restrict__ left, const uint32_t* __restrict__ cover,
+    lt_small_scan_kernel(uint32_t nodes, const uint32_t* left, const uint32_t* cover,
                          uint32_t* __restrict__ depth, uint32_t* __restrict__ wide, BuildControl* __restrict__ control)
 {
     __shared__ uint32_t s_cover[kSmallSortKeys];
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kSmallScanThreads)
 #pragma unroll
     for (int k = 0; k < kSmallScanItems; ++k) {
         const uint32_t i = first + k;
-        v[k] = i < nodes ? s_cover[__ldg(left + i) & ~kChildLeafBit] - 1u : 1u;
+        v[k] = i < nodes ? s_cover[chain_load(left + i) & ~kChildLeafBit] - 1u : 1u;
         deep = deep || (i < nodes && v[k] >= 128u);
         sum += (v[k] & 1u) == 0 ? 1u : 0u;
     }
@@ -631,10 +631,10 @@ __device__ __forceinline__ void row_word(uint32_t wd, uint32_t& c, uint32_t& idx
 
 __global__ void __launch_bounds__(kAggTile)
     lt_tile_kernel(uint32_t n, uint32_t node_capacity, LightSummary* __restrict__ sorted,
-                   const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
-                   const uint32_t* __restrict__ parent, const uint32_t* __restrict__ leaf_parent,
-                   const uint32_t* __restrict__ range_end, const uint32_t* __restrict__ depth,
-                   const uint32_t* __restrict__ wide, const uint32_t* __restrict__ values,
+                   const uint32_t* left, const uint32_t* right,
+                   const uint32_t* parent, const uint32_t* leaf_parent,
+                   const uint32_t* range_end, const uint32_t* depth,
+                   const uint32_t* wide, const uint32_t* values,
                    AggregateSlot* __restrict__ aggregates, uint32_t* __restrict__ upper,
                    uint32_t* __restrict__ crossing, LightBvhLeaf* __restrict__ leaves,
                    LightBvhNode* __restrict__ nodes, BuildControl* control)
@@ -682,17 +682,18 @@ __global__ void __launch_bounds__(kAggTile)
     if (j < n) {
         // The sorted leaf's summary, read through the permutation (the leaves' parent words,
         // written below by other tiles, are other bytes of the rows).
-        const uint32_t v = __ldg(values + j);
+        const uint32_t v = chain_load(values + j);
         s_value[k] = v;
         s_leaf[k] = load_summary(&leaves[v].summary);
-        node = __ldg(leaf_parent + j);
+        node = chain_load(leaf_parent + j);
     }
     if (j + 1 < n) {
-        const uint4 link = make_uint4(__ldg(left + j), __ldg(right + j), __ldg(parent + j), __ldg(range_end + j));
+        const uint4 link =
+            make_uint4(chain_load(left + j), chain_load(right + j), chain_load(parent + j), chain_load(range_end + j));
         s_link[k] = link;
-        s_wide[k] = __ldg(wide + j);
+        s_wide[k] = chain_load(wide + j);
         mine = min(j, link.w) >= lo && max(j, link.w) <= hi;
-        even = (__ldg(depth + j) & 1u) == 0;
+        even = (chain_load(depth + j) & 1u) == 0;
     }
     // The in-tile even-depth nodes in node order (their 4-wide indices rise with it); the block
     // scan's barriers also publish the loads above.
@@ -807,8 +808,9 @@ __global__ void __launch_bounds__(kAggTile)
                 uint32_t up_node = kNone, up_slot = 0;
                 if (i != 0) {
                     const auto link_of = [&](uint32_t x) {
-                        return x - lo < kAggTile ? s_link[x - lo]
-                                                 : make_uint4(__ldg(left + x), __ldg(right + x), __ldg(parent + x), 0u);
+                        return x - lo < kAggTile
+                                   ? s_link[x - lo]
+                                   : make_uint4(chain_load(left + x), chain_load(right + x), chain_load(parent + x), 0u);
                     };
                     const uint32_t p = link.z;
                     const uint4 lp = p + 1 < n ? link_of(p) : make_uint4(kNone, kNone, kNone, 0u);
@@ -817,7 +819,7 @@ __global__ void __launch_bounds__(kAggTile)
                         const uint32_t gl = link_of(g).x;
                         const uint32_t b0 = p == gl ? 0u : ((gl & kChildLeafBit) ? 1u : 2u);
                         up_slot = b0 + (lp.y == i ? 1u : 0u);
-                        up_node = g - lo < kAggTile ? s_wide[g - lo] : __ldg(wide + g);
+                        up_node = g - lo < kAggTile ? s_wide[g - lo] : chain_load(wide + g);
                     }
                 }
                 s_row[r * kNodeQuads + 13] = make_uint4(up_node, up_slot, 0u, 0u);
@@ -858,20 +860,20 @@ __device__ __forceinline__ LightSummary load_summary_weak(const LightSummary* p)
 
 // The walk from listed child `from`.
 template <bool kOneCta>
-__device__ __forceinline__ void upper_walk(uint32_t from, const LightSummary* __restrict__ sorted,
-                                           const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
-                                           const uint32_t* __restrict__ parent, const uint32_t* __restrict__ leaf_parent,
+__device__ __forceinline__ void upper_walk(uint32_t from, const LightSummary* sorted,
+                                           const uint32_t* left, const uint32_t* right,
+                                           const uint32_t* parent, const uint32_t* leaf_parent,
                                            uint32_t* counter, AggregateSlot* aggregates, BuildControl* control)
 {
     constexpr cuda::thread_scope kScope = kOneCta ? cuda::thread_scope_block : cuda::thread_scope_device;
     const bool leaf = (from & kChildLeafBit) != 0;
     LightSummary cur = leaf ? load_summary_cg(sorted + (from & ~kChildLeafBit)) : load_summary_cg(&aggregates[from].summary);
-    uint32_t node = leaf ? __ldg(leaf_parent + (from & ~kChildLeafBit)) : __ldg(parent + from);
+    uint32_t node = leaf ? chain_load(leaf_parent + (from & ~kChildLeafBit)) : chain_load(parent + from);
     uint32_t depth = 0;
     for (; depth < 128 && node != kNone; ++depth) {
-        const uint32_t l = __ldg(left + node);
-        const uint32_t r = __ldg(right + node);
-        const uint32_t up = __ldg(parent + node);
+        const uint32_t l = chain_load(left + node);
+        const uint32_t r = chain_load(right + node);
+        const uint32_t up = chain_load(parent + node);
         const uint32_t sibling = l == from ? r : l;
         cuda::atomic_ref<uint32_t, kScope> arrival(counter[node]);
         if (arrival.fetch_add(1u, cuda::memory_order_acq_rel) == 0) break;
@@ -888,10 +890,10 @@ __device__ __forceinline__ void upper_walk(uint32_t from, const LightSummary* __
 }
 
 __global__ void __launch_bounds__(kThreads)
-    lt_aggregate_upper_kernel(const LightSummary* __restrict__ sorted, const uint32_t* __restrict__ left,
-                              const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent,
-                              const uint32_t* __restrict__ leaf_parent, uint32_t* counter,
-                              AggregateSlot* aggregates, const uint32_t* __restrict__ upper, BuildControl* control)
+    lt_aggregate_upper_kernel(const LightSummary* sorted, const uint32_t* left,
+                              const uint32_t* right, const uint32_t* parent,
+                              const uint32_t* leaf_parent, uint32_t* counter,
+                              AggregateSlot* aggregates, const uint32_t* upper, BuildControl* control)
 {
     grid_wait();
     const uint32_t count = control->upper_count;
@@ -903,17 +905,17 @@ __global__ void __launch_bounds__(kThreads)
 // from the global arrays and slots, the row written by the thread; the parent words of its leaf slots
 // written into the leaves. count: the 4-wide nodes there is room for.
 template <bool kOneCta>
-__device__ __forceinline__ void upper_row(uint32_t i, uint32_t n, uint32_t count, const uint32_t* __restrict__ values,
-                                          const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
-                                          const uint32_t* __restrict__ parent, const uint32_t* __restrict__ wide,
-                                          const LightSummary* __restrict__ sorted, const AggregateSlot* aggregates,
+__device__ __forceinline__ void upper_row(uint32_t i, uint32_t n, uint32_t count, const uint32_t* values,
+                                          const uint32_t* left, const uint32_t* right,
+                                          const uint32_t* parent, const uint32_t* wide,
+                                          const LightSummary* sorted, const AggregateSlot* aggregates,
                                           LightBvhLeaf* __restrict__ leaves, LightBvhNode* __restrict__ nodes)
 {
-    const uint32_t w = __ldg(wide + i);
+    const uint32_t w = chain_load(wide + i);
     if (w >= count) return;
     uint32_t slots[4];
-    wide_slots(__ldg(left + i), __ldg(right + i),
-               [&](uint32_t x) { return make_uint2(__ldg(left + x), __ldg(right + x)); }, slots);
+    wide_slots(chain_load(left + i), chain_load(right + i),
+               [&](uint32_t x) { return make_uint2(chain_load(left + x), chain_load(right + x)); }, slots);
     uint4* row = reinterpret_cast<uint4*>(nodes + w);
     LightSummary sm[4];
     uint32_t word[4];
@@ -929,12 +931,12 @@ __device__ __forceinline__ void upper_row(uint32_t i, uint32_t n, uint32_t count
         if (slot & kChildLeafBit) {
             const uint32_t p = slot & ~kChildLeafBit;
             sm[c] = load_summary_cg(sorted + p);
-            const uint32_t leaf = __ldg(values + p);
+            const uint32_t leaf = chain_load(values + p);
             word[c] = kChildLeafBit | leaf;
             leaves[leaf].parent = (w << kParentSlotBits) | c;  // the leaf's parent word, in place
         } else {
             sm[c] = kOneCta ? load_summary_weak(&aggregates[slot].summary) : load_summary_cg(&aggregates[slot].summary);
-            word[c] = __ldg(wide + slot);
+            word[c] = chain_load(wide + slot);
         }
     }
     float f[48];
@@ -951,13 +953,13 @@ __device__ __forceinline__ void upper_row(uint32_t i, uint32_t n, uint32_t count
     // The node's own parent link.
     uint32_t up_node = kNone, up_slot = 0;
     if (i != 0) {
-        const uint32_t p = __ldg(parent + i);
-        const uint32_t g = p + 1 < n ? __ldg(parent + p) : kNone;
+        const uint32_t p = chain_load(parent + i);
+        const uint32_t g = p + 1 < n ? chain_load(parent + p) : kNone;
         if (g + 1 < n) {
-            const uint32_t gl = __ldg(left + g);
+            const uint32_t gl = chain_load(left + g);
             const uint32_t b0 = p == gl ? 0u : ((gl & kChildLeafBit) ? 1u : 2u);
-            up_slot = b0 + (__ldg(right + p) == i ? 1u : 0u);
-            up_node = __ldg(wide + g);
+            up_slot = b0 + (chain_load(right + p) == i ? 1u : 0u);
+            up_node = chain_load(wide + g);
         }
     }
     row[13] = make_uint4(up_node, up_slot, 0u, 0u);
@@ -966,12 +968,12 @@ __device__ __forceinline__ void upper_row(uint32_t i, uint32_t n, uint32_t count
 // The 4-wide nodes over the even-depth nodes that cross a tile (listed by the tile kernel): one thread
 // per node.
 __global__ void __launch_bounds__(kThreads)
-    lt_wide_upper_kernel(uint32_t n, uint32_t node_capacity, const uint32_t* __restrict__ values,
-                         const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
-                         const uint32_t* __restrict__ parent, const uint32_t* __restrict__ crossing,
-                         const uint32_t* __restrict__ wide, const LightSummary* __restrict__ sorted,
-                         const AggregateSlot* __restrict__ aggregates, LightBvhLeaf* __restrict__ leaves,
-                         LightBvhNode* __restrict__ nodes, const BuildControl* __restrict__ control)
+    lt_wide_upper_kernel(uint32_t n, uint32_t node_capacity, const uint32_t* values,
+                         const uint32_t* left, const uint32_t* right,
+                         const uint32_t* parent, const uint32_t* crossing,
+                         const uint32_t* wide, const LightSummary* sorted,
+                         const AggregateSlot* aggregates, LightBvhLeaf* __restrict__ leaves,
+                         LightBvhNode* __restrict__ nodes, const BuildControl* control)
 {
     grid_wait();
     const uint32_t count = min(control->node_count, node_capacity);
@@ -1060,7 +1062,7 @@ __global__ void __launch_bounds__(kScanThreads)
 // over boundary gamma are node i and its ancestors); even depths are flagged and scanned into the
 // 4-wide node index (wide[i]). The last tile writes the node count.
 __global__ void __launch_bounds__(kScanThreads)
-    lt_flags_scan_kernel(uint32_t nodes, const uint32_t* __restrict__ left, const uint32_t* __restrict__ cover,
+    lt_flags_scan_kernel(uint32_t nodes, const uint32_t* left, const uint32_t* cover,
                          uint32_t* __restrict__ depth_out, uint32_t* __restrict__ wide, uint32_t* states,
                          uint32_t* tile_counter, BuildControl* control)
 {
@@ -1076,7 +1078,7 @@ __global__ void __launch_bounds__(kScanThreads)
     uint32_t v[kScanItems];
     load_run(left, base, nodes, v);
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) v[k] = base + k < nodes ? __ldg(cover + (v[k] & ~kChildLeafBit)) - 1u : 0u;
+    for (int k = 0; k < kScanItems; ++k) v[k] = base + k < nodes ? chain_load(cover + (v[k] & ~kChildLeafBit)) - 1u : 0u;
     store_run(depth_out, base, nodes, v);
     uint32_t sum = 0;
     bool deep = false;
@@ -1170,11 +1172,11 @@ __global__ void lt_finish_kernel(uint32_t n, uint32_t found, uint32_t node_capac
 // the nodes that cross tiles, the header. One
 // launch for what are four in a larger build (18 us of the 4,096-leaf build's kernels in the place of 34).
 __global__ void __launch_bounds__(kTailThreads)
-    lt_tail_kernel(uint32_t n, uint32_t found, uint32_t node_capacity, const uint32_t* __restrict__ values,
-                   const LightSummary* __restrict__ sorted, const uint32_t* __restrict__ left,
-                   const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent,
-                   const uint32_t* __restrict__ leaf_parent, const uint32_t* __restrict__ wide, uint32_t* counter,
-                   AggregateSlot* aggregates, const uint32_t* __restrict__ upper, const uint32_t* __restrict__ crossing,
+    lt_tail_kernel(uint32_t n, uint32_t found, uint32_t node_capacity, const uint32_t* values,
+                   const LightSummary* sorted, const uint32_t* left,
+                   const uint32_t* right, const uint32_t* parent,
+                   const uint32_t* leaf_parent, const uint32_t* wide, uint32_t* counter,
+                   AggregateSlot* aggregates, const uint32_t* upper, const uint32_t* crossing,
                    LightBvhLeaf* __restrict__ leaves, LightBvhNode* __restrict__ nodes, LightTreeHeader* header,
                    LightTreeState* state, BuildControl* control)
 {

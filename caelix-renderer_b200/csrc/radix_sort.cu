@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) onesweep_pass_kernel(const So
 #pragma unroll
     for (int k = 0; k < KPT; ++k) {
         const uint32_t i = warp_base + k * 32u + lane;
-        key[k] = i < a.n ? __ldg(a.keys_in + i) : 0u;
+        key[k] = i < a.n ? chain_load(a.keys_in + i) : 0u;
     }
     warp_rank<KPT>(key, warp_base, a.n, a.shift, s_warp_counts[warp], pos);
     __syncthreads();
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) onesweep_pass_kernel(const So
 #pragma unroll
     for (int k = 0; k < KPT; ++k) {
         const uint32_t i = warp_base + k * 32u + lane;
-        if (i < a.n) s_values[pos.get(k)] = a.values_in ? __ldg(a.values_in + i) : i;
+        if (i < a.n) s_values[pos.get(k)] = a.values_in ? chain_load(a.values_in + i) : i;
     }
     __syncthreads();
     const uint32_t count = a.n - base < (uint32_t)kTile ? a.n - base : (uint32_t)kTile;
@@ -242,9 +242,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) onesweep_pass_kernel(const So
         if (a.rows_in) {
             const uint4* src = a.rows_in + (uint64_t)a.rows_in_stride * v;
             uint4* dst = a.rows_out + 3ull * dest;
-            const uint4 r0 = __ldg(src);
-            const uint4 r1 = __ldg(src + 1);
-            const uint4 r2 = __ldg(src + 2);
+            const uint4 r0 = chain_load(src);
+            const uint4 r1 = chain_load(src + 1);
+            const uint4 r2 = chain_load(src + 2);
             dst[0] = r0;
             dst[1] = r1;
             dst[2] = r2;
@@ -375,8 +375,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) onesweep_pipe_kernel(const So
         const uint32_t count = min(a.n - base, kPipeTile);
         const uint32_t bulk = ((count * 4u) & ~15u) / 4u;
         if (tid < count - bulk) {  // the last tile's tail (under 4 elements)
-            S.raw_keys[stage][bulk + tid] = __ldg(a.keys_in + base + bulk + tid);
-            if (a.values_in) S.raw_values[stage][bulk + tid] = __ldg(a.values_in + base + bulk + tid);
+            S.raw_keys[stage][bulk + tid] = chain_load(a.keys_in + base + bulk + tid);
+            if (a.values_in) S.raw_values[stage][bulk + tid] = chain_load(a.values_in + base + bulk + tid);
         }
         __syncthreads();
         const uint32_t warp_base = base + warp * 32u * KPT;
@@ -433,9 +433,9 @@ __global__ void __launch_bounds__(kSortThreads, 2) onesweep_pipe_kernel(const So
             if (a.rows_in) {
                 const uint4* src = a.rows_in + (uint64_t)a.rows_in_stride * v;
                 uint4* dst = a.rows_out + 3ull * dest;
-                const uint4 r0 = __ldg(src);
-                const uint4 r1 = __ldg(src + 1);
-                const uint4 r2 = __ldg(src + 2);
+                const uint4 r0 = chain_load(src);
+                const uint4 r1 = chain_load(src + 1);
+                const uint4 r2 = chain_load(src + 2);
                 dst[0] = r0;
                 dst[1] = r1;
                 dst[2] = r2;
@@ -519,9 +519,9 @@ __global__ void __launch_bounds__(kSortThreads) small_sort_kernel(uint32_t* __re
         if (gather.rows_in) {
             const uint4* src = gather.rows_in + (uint64_t)gather.rows_in_stride * v;
             uint4* dst = gather.rows_out + 3ull * i;
-            dst[0] = __ldg(src);
-            dst[1] = __ldg(src + 1);
-            dst[2] = __ldg(src + 2);
+            dst[0] = chain_load(src);
+            dst[1] = chain_load(src + 1);
+            dst[2] = chain_load(src + 2);
             if (gather.inverse) gather.inverse[v] = i;
         }
     }
@@ -559,9 +559,9 @@ __global__ void __launch_bounds__(kSortThreads) rank_sort_kernel(uint32_t* __res
         if (gather.rows_in) {
             const uint4* src = gather.rows_in + (uint64_t)gather.rows_in_stride * v;
             uint4* dst = gather.rows_out + 3ull * r;
-            dst[0] = __ldg(src);
-            dst[1] = __ldg(src + 1);
-            dst[2] = __ldg(src + 2);
+            dst[0] = chain_load(src);
+            dst[1] = chain_load(src + 1);
+            dst[2] = chain_load(src + 2);
             if (gather.inverse) gather.inverse[v] = r;
         }
     }
