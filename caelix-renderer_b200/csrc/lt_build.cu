@@ -838,12 +838,19 @@ __global__ void __launch_bounds__(kAggTile)
 // The walks up through the nodes whose range crosses a tile, from the children the tiles listed
 // (an in-tile node, its summary in its slot, or a leaf): the second thread to arrive at a node
 // computes it and goes on. The walks were run inside the tile kernel at first: chains of
-// dependent device-scope atomics and L2 loads that kept each tile's CTA resident for them. Builds of
-// up to kTailLeaves leaves run them in one CTA (kOneCta), whose arrivals are block-scope and whose
-// siblings' summaries come through L1; larger ones on a persistent grid with device-scope arrivals.
-// With six walks per thread (97 k leaves) the one CTA was slower than the grid (the light-tree flush of
-// the 2 M-brick world 0.22 against 0.18 ms).
-constexpr uint32_t kTailLeaves = 16384;
+// dependent device-scope atomics and L2 loads that kept each tile's CTA resident for them. Up to kTailThreads
+// walks (one per thread: about 32,000 leaves) run in one CTA (kOneCta), whose arrivals are block-scope and
+// whose siblings' summaries come through L1; more on a persistent grid with device-scope arrivals. The rows and
+// the header that follow are the one CTA's work too (lt_tail_kernel) in builds of up to kTailLeaves leaves. In
+// those of up to kOneCtaLeaves both variants are launched and one returns at once: how many walks there are
+// is known on the device only, and depends on where the lights are. Larger ones launch the grid alone. Whole builds
+// in us (one B200, lights uniform in a box): the tail / both variants / the grid alone,
+//    6,000 leaves 103 / 105 / 112      24,000  123.5 / 124.4 / 129.7     36,000  142 / 131.6 / 131.2
+//   16,385        117 / 119 / 126      28,000  125.5 / 124.5 / 128.8     48,000  151 / 137.2 / 136.1
+//   20,000        121 / 122 / 127      32,000  128.4 / 127.0 / 131.0     64,000  163 / 140.2 / 139.5
+// and lights on a line (few walks) 48,000 117 / 119 / 123, in eight clusters 28,000 132 / 131 / 137.
+constexpr uint32_t kTailLeaves = 24576;
+constexpr uint32_t kOneCtaLeaves = 65536;
 constexpr uint32_t kTailThreads = 1024;
 
 // A summary written earlier by this kernel's CTA (after an acquire: weak loads through L1).
@@ -889,16 +896,19 @@ __device__ __forceinline__ void upper_walk(uint32_t from, const LightSummary* so
     if (depth == 128) atomicOr(&control->status, kStatusDepthGuard);
 }
 
-__global__ void __launch_bounds__(kThreads)
+// few: the launch is for up to (kOneCta) or above so many walks; the list's length is known on the device only.
+template <bool kOneCta>
+__global__ void __launch_bounds__(kOneCta ? kTailThreads : kThreads)
     lt_aggregate_upper_kernel(const LightSummary* sorted, const uint32_t* left,
                               const uint32_t* right, const uint32_t* parent,
                               const uint32_t* leaf_parent, uint32_t* counter,
-                              AggregateSlot* aggregates, const uint32_t* upper, BuildControl* control)
+                              AggregateSlot* aggregates, const uint32_t* upper, BuildControl* control, uint32_t few)
 {
     grid_wait();
     const uint32_t count = control->upper_count;
+    if (kOneCta ? count > few : count <= few) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-        upper_walk<false>(upper[i], sorted, left, right, parent, leaf_parent, counter, aggregates, control);
+        upper_walk<kOneCta>(upper[i], sorted, left, right, parent, leaf_parent, counter, aggregates, control);
 }
 
 // The 4-wide node over even-depth binary node i, which crosses a tile: children and summaries read
@@ -1169,8 +1179,7 @@ __global__ void lt_finish_kernel(uint32_t n, uint32_t found, uint32_t node_capac
 }
 
 // After the tile kernel of a build of 2 to kTailLeaves leaves, by one CTA: the upper walks, the rows over
-// the nodes that cross tiles, the header. One
-// launch for what are four in a larger build (18 us of the 4,096-leaf build's kernels in the place of 34).
+// the nodes that cross tiles, the header: one launch for what are three or four in a larger build.
 __global__ void __launch_bounds__(kTailThreads)
     lt_tail_kernel(uint32_t n, uint32_t found, uint32_t node_capacity, const uint32_t* values,
                    const LightSummary* sorted, const uint32_t* left,
@@ -1365,9 +1374,14 @@ cudaError_t lt_build(const LightBvhBuffers& b, const LightBvhInput& in, cudaStre
             mark(7);
             return e != cudaSuccess ? e : cudaGetLastError();
         }
+        const uint32_t few = n <= kOneCtaLeaves ? kTailThreads : 0u;
+        if (e == cudaSuccess && few)
+            e = launch_chained(lt_aggregate_upper_kernel<true>, 1, kTailThreads, 0, stream, b.sorted, b.left, b.right,
+                               b.parent, b.leaf_parent, b.counter, b.aggregates, b.cover, b.control, few);
         if (e == cudaSuccess)
-            e = launch_chained(lt_aggregate_upper_kernel, grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream, b.sorted,
-                               b.left, b.right, b.parent, b.leaf_parent, b.counter, b.aggregates, b.cover, b.control);
+            e = launch_chained(lt_aggregate_upper_kernel<false>, grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream,
+                               b.sorted, b.left, b.right, b.parent, b.leaf_parent, b.counter, b.aggregates, b.cover,
+                               b.control, few);
         mark(6);
         if (e == cudaSuccess)
             e = launch_chained(lt_wide_upper_kernel, grid_for(nodes, kThreads, sms * 8), kThreads, 0, stream, n,
@@ -1391,12 +1405,12 @@ cudaError_t lt_build(const LightBvhBuffers& b, const LightBvhInput& in, cudaStre
 
 uint32_t lt_kernel_launches(uint32_t n)
 {
-    // finish; emit, Morton, sort, finish; emit, keys, sort, Karras, scan, tile,
-    // tail; emit, Morton, four sort passes, Karras, two
-    // scans, tile, then the tail, or upper aggregation, upper rows and finish.
+    // finish; emit, Morton, sort, finish; emit, keys, sort, Karras, scan, tile, tail; emit, Morton, four sort
+    // passes, Karras, two scans, tile, then the tail, or upper aggregation (both variants up to kOneCtaLeaves),
+    // upper rows and finish.
     if (n <= 1) return n == 0 ? 1u : 4u;
     if (n <= kSmallSortKeys) return 7;
-    return 10u + (n <= kTailLeaves ? 1u : 3u);
+    return 10u + (n <= kTailLeaves ? 1u : n <= kOneCtaLeaves ? 4u : 3u);
 }
 
 }  // namespace cx

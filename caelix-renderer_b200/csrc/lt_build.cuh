@@ -4,7 +4,7 @@
 //
 // Replaces the reference's per-tree dispatch sequence LightTree::RecordTree
 // (lib/src/light/light_tree_record.cpp:230-309, about 35 dependent dispatches with a barrier after
-// each) with 13 kernels and one memset (11 up to 16,384 leaves, 7 up to 4,096), the kernels' launches
+// each) with 13 kernels and one memset (14 up to 65,536 leaves, 11 up to 24,576, 7 up to 4,096), the kernels' launches
 // chained (launch.cuh), all on one stream (capturable in a CUDA graph):
 //   lt_emit_kernel        gather emit (caelix_light_gather_emit.hlsl:11-86) fused with the centre
 //                         bounds (caelix_light_bvh_bounds.hlsl:10-53): warp max-reductions of
@@ -22,10 +22,11 @@
 //   lt_tile_kernel        by tiles of 256 sorted leaves in shared memory: the aggregation
 //                         (caelix_light_bvh_aggregate.hlsl:30-55) of the nodes inside the tile and
 //                         the 4-wide nodes over them (caelix_light_bvh_wide.hlsl:10-100)
-//   lt_aggregate_upper_kernel  the aggregation of the nodes that cross tiles (acq_rel arrivals)
+//   lt_aggregate_upper_kernel  the aggregation of the nodes that cross tiles (acq_rel arrivals; up to
+//                         65,536 leaves two variants, one CTA for few walks or a persistent grid)
 //   lt_wide_upper_kernel  the 4-wide nodes over the nodes that cross tiles
 //   lt_finish_kernel      caelix_light_bvh_finish.hlsl:8-63
-// Up to 16,384 leaves lt_tail_kernel does the work of the last three in one CTA; up to 4,096
+// Up to 24,576 leaves lt_tail_kernel does the work of the last three in one CTA; up to 4,096
 // lt_small_keys_kernel, lt_rank_sort_kernel, lt_small_karras_kernel and lt_small_scan_kernel take the
 // places of Morton, sort, Karras and the scans.
 // Every float operation is a single IEEE fp32 operation in the order of the HLSL source (the
