@@ -63,26 +63,6 @@ CaelixResult status_result(uint32_t status, const char* what)
     return CAELIX_ERROR_DEVICE_STATUS;
 }
 
-// Device memory grown on demand (never shrunk).
-CaelixResult GrowBuffer::reserve(uint64_t want, const char* what)
-{
-    if (want <= bytes) return CAELIX_OK;
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-    const cudaError_t e = cudaMalloc(&ptr, want);
-    if (e != cudaSuccess) return cuda_result(e, what);
-    bytes = want;
-    return CAELIX_OK;
-}
-
-void GrowBuffer::release()
-{
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-}
-
 }  // namespace cx
 
 struct CaelixLightBvh

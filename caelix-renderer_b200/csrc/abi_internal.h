@@ -6,6 +6,7 @@
 #include <new>
 
 #include "../../include/caelix_b200.h"
+#include "grow_buffer.h"
 
 // Exceptions never cross the C ABI: the body of every entry point that may allocate on the host
 // runs inside CAELIX_GUARD_BEGIN / CAELIX_GUARD_END.
@@ -28,17 +29,6 @@ namespace cx {
 void log(CaelixLogLevel level, const char* fmt, ...);
 CaelixResult cuda_result(cudaError_t e, const char* what);
 CaelixResult status_result(uint32_t status, const char* what);
-
-// Device memory grown on demand (never shrunk); freed by release().
-struct GrowBuffer
-{
-    void* ptr = nullptr;
-    uint64_t bytes = 0;
-    CaelixResult reserve(uint64_t want, const char* what);
-    // reserve, growing by an extra eighth when it has to grow (buffers sized by a scene).
-    CaelixResult reserve_grow(uint64_t want, const char* what) { return want <= bytes ? CAELIX_OK : reserve(want + want / 8, what); }
-    void release();
-};
 
 }  // namespace cx
 

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <unordered_map>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "../../include/caelix_b200.h"
@@ -1276,7 +1277,7 @@ CAELIX_API void caelix_renderer_destroy(CaelixRenderer* renderer)
     if (renderer->counts) cudaFree(renderer->counts);
     if (renderer->start) cudaEventDestroy(renderer->start);
     if (renderer->stop) cudaEventDestroy(renderer->stop);
-    renderer->wave_memory.release();
+    renderer->wave_memory.buffer.release();
     renderer->wave_views.release();
     delete renderer;
 }
@@ -1316,14 +1317,17 @@ CAELIX_API CaelixResult caelix_renderer_render(CaelixRenderer* renderer, const C
         const auto slots_of = [&](const cx::WavePlan& w) {
             return renderer->wave_capacity ? std::min(renderer->wave_capacity, w.largest()) : w.largest();
         };
-        CaelixResult r2 =
-            renderer->wave_memory.reserve(cx::wave_buffer_bytes(slots_of(plan)), "caelix_renderer_render");
-        if (r2 == CAELIX_ERROR_OUT_OF_MEMORY) {
-            // One sample index per wave where the path state of several does not fit.
-            cudaGetLastError();
-            plan = cx::wave_plan(&view, 1, kBlockWidth, 0);
-            r2 = renderer->wave_memory.reserve(cx::wave_buffer_bytes(slots_of(plan)), "caelix_renderer_render");
-        }
+        // One sample index per wave where the path state of several does not fit.
+        cx::WavePlan single;
+        bool merged = false;
+        CaelixResult r2 = renderer->wave_memory.reserve(
+            cx::wave_buffer_bytes(slots_of(plan)),
+            [&] {
+                single = cx::wave_plan(&view, 1, kBlockWidth, 0);
+                return cx::wave_buffer_bytes(slots_of(single));
+            },
+            "caelix_renderer_render", &merged);
+        if (!merged) plan = std::move(single);
         const uint32_t capacity = slots_of(plan);
         const uint64_t view_bytes = (sizeof(cx::WaveView) + 255) & ~uint64_t{255};
         if (r2 == CAELIX_OK)
@@ -1336,7 +1340,7 @@ CAELIX_API CaelixResult caelix_renderer_render(CaelixRenderer* renderer, const C
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_table, plan.table.data(), 4 * plan.table.size(), cudaMemcpyHostToDevice, stream);
         if (e != cudaSuccess) return cx::cuda_result(e, "caelix_renderer_render");
-        const cx::WaveBuffers wb = cx::wave_carve(renderer->wave_memory.ptr, capacity);
+        const cx::WaveBuffers wb = cx::wave_carve(renderer->wave_memory.buffer.ptr, capacity);
         renderer->launches = 0;
         cudaEventRecord(renderer->start, stream);
         e = cx::wave_trace(&view, d_view, 1, plan, d_table, wb, kBlockWidth, renderer->device->sm_count, stream,
@@ -1372,20 +1376,18 @@ CAELIX_API CaelixResult caelix_renderer_backward(CaelixRenderer* renderer, const
     if (e == cudaSuccess) e = cudaMemsetAsync(d_power, 0, sizeof(float) * std::max(scene->dev.brick_count, 1u), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(renderer->counts, 0, 24, stream);
     if (e != cudaSuccess) return cx::cuda_result(e, "caelix_renderer_backward");
+    // One sample index per wave where the path state of several does not fit.
     uint32_t merge = cx::wave_merge_slots(renderer->wave_capacity);
-    CaelixResult r2 =
-        renderer->wave_memory.reserve(cx::adjoint_bytes(p, renderer->wave_capacity, merge), "caelix_renderer_backward");
-    if (r2 == CAELIX_ERROR_OUT_OF_MEMORY) {
-        // One sample index per wave where the path state of several does not fit.
-        cudaGetLastError();
-        merge = 0;
-        r2 = renderer->wave_memory.reserve(cx::adjoint_bytes(p, renderer->wave_capacity, merge), "caelix_renderer_backward");
-    }
+    bool merged = false;
+    const CaelixResult r2 = renderer->wave_memory.reserve(
+        cx::adjoint_bytes(p, renderer->wave_capacity, merge),
+        [&] { return cx::adjoint_bytes(p, renderer->wave_capacity, 0); }, "caelix_renderer_backward", &merged);
+    if (!merged) merge = 0;
     if (r2 != CAELIX_OK) return r2;
     renderer->launches = 0;
     cudaEventRecord(renderer->start, stream);
     e = cx::adjoint_launch(render_view(scene), p, d_radiance, reinterpret_cast<float*>(image), d_albedo,
-                           d_power, renderer->counts, renderer->wave_memory.ptr, renderer->wave_capacity,
+                           d_power, renderer->counts, renderer->wave_memory.buffer.ptr, renderer->wave_capacity,
                            merge, renderer->device->sm_count, stream, &renderer->launches);
     cudaEventRecord(renderer->stop, stream);
     renderer->last_stream = stream;
@@ -1402,6 +1404,7 @@ CAELIX_API CaelixResult caelix_renderer_set_trace_mode(CaelixRenderer* renderer,
         return CAELIX_ERROR_INVALID_ARGUMENT;
     renderer->trace_mode = mode;
     renderer->wave_capacity = wave_capacity;
+    renderer->wave_memory.forget();
     return CAELIX_OK;
 }
 

@@ -133,7 +133,7 @@ struct CaelixRenderer
     bool rendered = false;
     uint32_t trace_mode = 0;        // CAELIX_TRACE_WAVEFRONT or CAELIX_TRACE_MEGAKERNEL
     uint32_t wave_capacity = 0;     // bounds the paths in flight (0: the wave plan's slots)
-    cx::GrowBuffer wave_memory;     // path state and queues of the wavefront trace
+    cx::WaveMemory wave_memory;     // path state and queues of the wavefront trace
     cx::GrowBuffer wave_views;      // the device copy of the view and its wave table
     uint32_t launches = 0;          // kernels of the newest render
 };

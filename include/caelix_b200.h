@@ -581,8 +581,9 @@ CAELIX_API CaelixResult caelix_renderer_render(CaelixRenderer* renderer, const C
    for bit.
      CAELIX_TRACE_WAVEFRONT (default): path state in device memory, one kernel per stage (trace,
        shade) over compacted ray and path queues, every bounce; wave_capacity bounds the paths in
-       flight (0 = one per pixel, or one per pixel and sample while that is at most 2^23; else at
-       least 32), the rest of the pixels and samples follow in later waves.
+       flight (0 = one per pixel, or one per pixel and sample while that is at most 2^23 and its path
+       state fits the device; else at least 32), the rest of the pixels and samples follow in later
+       waves. A size that did not fit is not asked for again until the mode is set again.
      CAELIX_TRACE_MEGAKERNEL: one thread per pixel runs its whole path in one kernel. */
 #define CAELIX_TRACE_WAVEFRONT 0u
 #define CAELIX_TRACE_MEGAKERNEL 1u
