@@ -121,9 +121,15 @@ CaelixBatchTuning run_tuning(const CaelixBatch* b)
     return t;
 }
 
-void release(CaelixBatch* b)
+void drop_graph(CaelixBatch* b)
 {
     if (b->exec) cudaGraphExecDestroy(b->exec);
+    b->exec = nullptr;
+}
+
+void release(CaelixBatch* b)
+{
+    drop_graph(b);
     if (b->d_views) cudaFree(b->d_views);
     if (b->d_wave_views) cudaFree(b->d_wave_views);
     b->wave_table.release();
@@ -141,9 +147,11 @@ void release(CaelixBatch* b)
 }
 
 // The device view table for a tuning: views ordered as the tuning says, consecutive item ranges,
-// counters by the caller's view index. Uploaded synchronously (outside any capture).
+// counters by the caller's view index. Uploaded synchronously (outside any capture). The captured graph
+// goes: it reads these tables, and path state that may move here, and is right for its own tuning's only.
 cudaError_t upload_views(CaelixBatch* b, const CaelixBatchTuning& t, uint32_t* item_count)
 {
+    drop_graph(b);
     const uint32_t n = (uint32_t)b->views.size();
     std::vector<uint32_t> order(n);
     for (uint32_t i = 0; i < n; ++i) order[i] = i;
@@ -316,10 +324,6 @@ cudaError_t ensure_graph(CaelixBatch* b)
         if (!s->built) return cudaErrorInvalidValue;
     // The view table is rewritten below: the previous run must have finished reading it.
     if (b->ran) CX_TRY(cudaStreamSynchronize(b->last_stream));
-    if (b->exec) {
-        cudaGraphExecDestroy(b->exec);
-        b->exec = nullptr;
-    }
     b->graph_tuning = t;
     uint32_t kernels = 0;
     cudaError_t e = capture_graph(b, t, true, true, &b->exec, &kernels);
