@@ -15,6 +15,7 @@
 #include <fstream>
 #include <sstream>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/caelix_b200.h"
@@ -75,7 +76,7 @@ struct CaelixBatch
     cx::BatchView* d_views = nullptr;
     cx::WaveView* d_wave_views = nullptr;
     cx::GrowBuffer wave_table;               // the wave plan's view tables
-    cx::GrowBuffer wave_memory;              // path state and queues of the wavefront kernels
+    cx::WaveMemory wave_memory;              // path state and queues of the wavefront kernels
     cx::WavePlan plan;                       // of the uploaded view order
     std::vector<cx::WaveView> wave_views;    // host copy, in the uploaded order
     unsigned long long* d_counts = nullptr;  // [view][3]
@@ -133,7 +134,7 @@ void release(CaelixBatch* b)
     if (b->d_views) cudaFree(b->d_views);
     if (b->d_wave_views) cudaFree(b->d_wave_views);
     b->wave_table.release();
-    b->wave_memory.release();
+    b->wave_memory.buffer.release();
     if (b->d_counts) cudaFree(b->d_counts);
     if (b->d_next) cudaFree(b->d_next);
     if (b->capture) cudaStreamDestroy(b->capture);
@@ -198,13 +199,22 @@ cudaError_t upload_views(CaelixBatch* b, const CaelixBatchTuning& t, uint32_t* i
     CX_TRY(cudaMemcpy(b->d_wave_views, b->wave_views.data(), sizeof(cx::WaveView) * n, cudaMemcpyHostToDevice));
     const uint32_t most = t.wavefront ? t.wavefront : kDefaultWaveSlots;
     b->plan = cx::wave_plan(b->wave_views.data(), n, bw, most);
+    const auto slots_of = [&](const cx::WavePlan& w) { return std::min(w.largest(), most); };
+    // One sample index per wave where the path state of several does not fit.
+    cx::WavePlan single;
+    bool merged = false;
+    const CaelixResult r = b->wave_memory.reserve(
+        cx::wave_buffer_bytes(slots_of(b->plan)),
+        [&] {
+            single = cx::wave_plan(b->wave_views.data(), n, bw, 0);
+            return cx::wave_buffer_bytes(slots_of(single));
+        },
+        "caelix_batch_run", &merged);
+    if (r != CAELIX_OK) return cudaErrorMemoryAllocation;
+    if (!merged) b->plan = std::move(single);
     if (b->wave_table.reserve(4ull * std::max<size_t>(b->plan.table.size(), 1), "caelix_batch_run") != CAELIX_OK)
         return cudaErrorMemoryAllocation;
-    CX_TRY(cudaMemcpy(b->wave_table.ptr, b->plan.table.data(), 4 * b->plan.table.size(), cudaMemcpyHostToDevice));
-    const uint32_t slots = std::min(b->plan.largest(), most);
-    if (b->wave_memory.reserve(cx::wave_buffer_bytes(slots), "caelix_batch_run") != CAELIX_OK)
-        return cudaErrorMemoryAllocation;
-    return cudaSuccess;
+    return cudaMemcpy(b->wave_table.ptr, b->plan.table.data(), 4 * b->plan.table.size(), cudaMemcpyHostToDevice);
 }
 
 uint32_t wave_slots(const CaelixBatch* b, const CaelixBatchTuning& t)
@@ -254,7 +264,7 @@ cudaError_t record(CaelixBatch* b, const CaelixBatchTuning& t, uint32_t item_cou
     }
     if (trace && run_kernel(b, t) == CAELIX_BATCH_WAVEFRONT) {
         CX_TRY(cudaMemsetAsync(b->d_counts, 0, 24ull * b->views.size(), s));
-        const cx::WaveBuffers wb = cx::wave_carve(b->wave_memory.ptr, wave_slots(b, t));
+        const cx::WaveBuffers wb = cx::wave_carve(b->wave_memory.buffer.ptr, wave_slots(b, t));
         return cx::wave_trace(b->wave_views.data(), b->d_wave_views, (uint32_t)b->views.size(), b->plan,
                               static_cast<const uint32_t*>(b->wave_table.ptr), wb, t.block_width, b->device->sm_count,
                               s, nullptr);
@@ -593,6 +603,7 @@ CAELIX_API CaelixResult caelix_batch_set_tuning(CaelixBatch* batch, const Caelix
     if (!batch || !tuning || !tuning_ok(*tuning)) return CAELIX_ERROR_INVALID_ARGUMENT;
     batch->tuning = *tuning;
     batch->tuned = true;
+    batch->wave_memory.forget();
     return CAELIX_OK;
 }
 
