@@ -21,6 +21,7 @@
 #include "../../include/caelix_b200.h"
 #include "abi_internal.h"
 #include "abi_scene_internal.h"
+#include "batch_tuning.h"
 #include "lt_build.cuh"
 #include "scene.cuh"
 #include "trace.cuh"
@@ -56,11 +57,6 @@ bool tuning_ok(const CaelixBatchTuning& t)
            t.reserved == 0;
 }
 
-bool same_tuning(const CaelixBatchTuning& a, const CaelixBatchTuning& b)
-{
-    return std::memcmp(&a, &b, sizeof(a)) == 0;
-}
-
 }  // namespace
 
 struct CaelixBatch
@@ -71,8 +67,7 @@ struct CaelixBatch
     std::vector<CaelixScene*> scenes;       // distinct scenes, in order of first appearance
     std::vector<uint64_t> generations;      // of the scenes when the graph was captured
     std::vector<uint64_t> entity_generations;  // of the scenes' entity views then
-    CaelixBatchTuning tuning = default_tuning();
-    bool tuned = false;  // the tuning was set or autotuned
+    BatchTuning tuning{default_tuning()};
     cx::BatchView* d_views = nullptr;
     cx::WaveView* d_wave_views = nullptr;
     cx::GrowBuffer wave_table;               // the wave plan's view tables
@@ -86,7 +81,6 @@ struct CaelixBatch
     cudaEvent_t fork = nullptr;
     cudaEvent_t joins[kMaxBranches] = {};
     cudaGraphExec_t exec = nullptr;
-    CaelixBatchTuning graph_tuning{};  // the tuning `exec` was captured for (run_tuning)
     uint32_t captures = 0;
     uint32_t kernel_nodes = 0;
     uint32_t wavefront = 0;
@@ -105,21 +99,6 @@ uint32_t run_kernel(const CaelixBatch* b, const CaelixBatchTuning& t)
     for (const CaelixScene* s : b->scenes)
         if (s->entity_view_count) return CAELIX_BATCH_WAVEFRONT;
     return t.kernel;
-}
-
-// The tuning a run uses: the batch's, or while none was set or autotuned the wavefront kernels over
-// 8 x 4 pixel blocks. Those are the faster organisation at every size measured (one B200, persistent
-// against wavefront kernels): one view of 32 x 32 0.160 / 0.133 ms, 4 views of 64 and 128 squared
-// 0.430 / 0.357, 12 views of 256 and 512 squared with 2 spp 17.0 / 5.84, 8 views of scenes of up to
-// 200 k bricks 12.5 / 4.57 (1 spp to 2 spp, 2 to 4 bounces).
-CaelixBatchTuning run_tuning(const CaelixBatch* b)
-{
-    CaelixBatchTuning t = b->tuning;
-    if (!b->tuned) {
-        t.kernel = CAELIX_BATCH_WAVEFRONT;
-        t.block_width = 8;
-    }
-    return t;
 }
 
 void drop_graph(CaelixBatch* b)
@@ -328,23 +307,21 @@ bool scenes_moved(const CaelixBatch* b)
 // The graph of a full run with the batch's tuning, captured again when needed.
 cudaError_t ensure_graph(CaelixBatch* b)
 {
-    CaelixBatchTuning t = run_tuning(b);
-    if (b->exec && same_tuning(b->graph_tuning, t) && !scenes_moved(b)) return cudaSuccess;
+    if (b->exec && b->tuning.serves() && !scenes_moved(b)) return cudaSuccess;
     for (CaelixScene* s : b->scenes)
         if (!s->built) return cudaErrorInvalidValue;
     // The view table is rewritten below: the previous run must have finished reading it.
     if (b->ran) CX_TRY(cudaStreamSynchronize(b->last_stream));
-    b->graph_tuning = t;
     uint32_t kernels = 0;
-    cudaError_t e = capture_graph(b, t, true, true, &b->exec, &kernels);
-    if (e == cudaErrorMemoryAllocation && !b->tuned) {
-        // No room for the paths' state: the persistent kernel keeps it in registers.
+    cudaError_t e = capture_graph(b, b->tuning.run(), true, true, &b->exec, &kernels);
+    if (e == cudaErrorMemoryAllocation && b->tuning.give_way()) {
         cudaGetLastError();
-        t = b->tuning;
-        e = capture_graph(b, t, true, true, &b->exec, &kernels);
+        e = capture_graph(b, b->tuning.run(), true, true, &b->exec, &kernels);
     }
     if (e != cudaSuccess) return e;
+    b->tuning.captured();
     b->kernel_nodes = kernels;
+    const CaelixBatchTuning t = b->tuning.run();
     b->wavefront = run_kernel(b, t) == CAELIX_BATCH_WAVEFRONT ? wave_slots(b, t) : trace_grid(b, t) * cx::kBatchThreads;
     for (size_t i = 0; i < b->scenes.size(); ++i) {
         b->generations[i] = b->scenes[i]->generation;
@@ -601,8 +578,7 @@ CAELIX_API CaelixResult caelix_batch_run(CaelixBatch* batch, const CaelixFrameDe
 CAELIX_API CaelixResult caelix_batch_set_tuning(CaelixBatch* batch, const CaelixBatchTuning* tuning)
 {
     if (!batch || !tuning || !tuning_ok(*tuning)) return CAELIX_ERROR_INVALID_ARGUMENT;
-    batch->tuning = *tuning;
-    batch->tuned = true;
+    batch->tuning.set(*tuning);
     batch->wave_memory.forget();
     return CAELIX_OK;
 }
@@ -610,7 +586,7 @@ CAELIX_API CaelixResult caelix_batch_set_tuning(CaelixBatch* batch, const Caelix
 CAELIX_API CaelixResult caelix_batch_get_tuning(const CaelixBatch* batch, CaelixBatchTuning* out)
 {
     if (!batch || !out) return CAELIX_ERROR_INVALID_ARGUMENT;
-    *out = batch->tuning;
+    *out = batch->tuning.own;
     return CAELIX_OK;
 }
 
@@ -623,10 +599,9 @@ CAELIX_API CaelixResult caelix_batch_autotune(CaelixBatch* batch, const CaelixFr
     for (CaelixScene* s : batch->scenes)
         if (!s->built) return CAELIX_ERROR_INVALID_ARGUMENT;
     const std::string key = tuning_key(batch);
-    CaelixBatchTuning t = batch->tuning;
+    CaelixBatchTuning t = batch->tuning.own;
     if (cache_path && cache_lookup(cache_path, key, &t)) {
-        batch->tuning = t;
-        batch->tuned = true;
+        batch->tuning.set(t);
         if (out) *out = t;
         return CAELIX_OK;
     }
@@ -701,8 +676,7 @@ CAELIX_API CaelixResult caelix_batch_autotune(CaelixBatch* batch, const CaelixFr
         }
     }
     t = best_t;
-    batch->tuning = t;
-    batch->tuned = true;
+    batch->tuning.set(t);
     if (cache_path && !cache_store(cache_path, key, t, best))
         log(CAELIX_LOG_WARNING, "caelix_batch_autotune: could not write the cache %s", cache_path);
     if (out) *out = t;
