@@ -53,7 +53,7 @@ uint64_t adjoint_bytes(const TraceParams& p, uint32_t wave_capacity, uint32_t me
     const WavePlan plan = wave_plan(&v, 1, kAdjointBlockWidth, merge_slots);
     const uint32_t capacity = plan_capacity(plan, wave_capacity);
     return 2 * align256(sizeof(WaveView)) + align256(4ull * plan.table.size()) +
-           align256(12ull * p.spp * p.width * p.height) + wave_buffer_bytes(capacity);
+           align256(12ull * p.spp * p.width * p.height) + wave_buffer_bytes(capacity, true);
 }
 
 cudaError_t adjoint_launch(const SceneView& s, const TraceParams& p, const float* d_radiance, float* image,
@@ -82,7 +82,7 @@ cudaError_t adjoint_launch(const SceneView& s, const TraceParams& p, const float
     m += align256(4ull * plan.table.size());
     float* samples = reinterpret_cast<float*>(m);
     m += align256(12ull * p.spp * p.width * p.height);
-    const WaveBuffers wb = wave_carve(m, capacity);
+    const WaveBuffers wb = wave_carve(m, capacity, true);
     CX_TRY(cudaMemcpyAsync(d_record, &views[0], sizeof(WaveView), cudaMemcpyHostToDevice, stream));
     CX_TRY(cudaMemcpyAsync(d_replay, &views[1], sizeof(WaveView), cudaMemcpyHostToDevice, stream));
     CX_TRY(cudaMemcpyAsync(d_table, plan.table.data(), 4 * plan.table.size(), cudaMemcpyHostToDevice, stream));

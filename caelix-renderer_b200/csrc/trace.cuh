@@ -111,8 +111,9 @@ struct WaveAdjoint
     float* d_power;   // [brick_count]
 };
 
-uint64_t wave_buffer_bytes(uint32_t capacity);
-WaveBuffers wave_carve(void* base, uint32_t capacity);
+// adjoint: with the adjoint's arrays (wave_adjoint; a plain render has none).
+uint64_t wave_buffer_bytes(uint32_t capacity, bool adjoint = false);
+WaveBuffers wave_carve(void* base, uint32_t capacity, bool adjoint = false);
 
 // The wave plan of a set of views. A wave holds the samples [first, first + samples) of the views
 // with spp > first (every one of them has all these samples): its entries are (view, sample) pairs,
@@ -125,7 +126,7 @@ WaveBuffers wave_carve(void* base, uint32_t capacity);
 // index against several in one wave: 333 x 251, 8 spp 3.65 against 1.48 ms; the adjoint of 256 x 256,
 // 8 spp 7.60 against 3.83 ms; 1920 x 1080, 4 spp (8.3 M paths at once) 25.5 against 20.4 ms. Fewer
 // slots: 1.78 ms for the first at 512 k (two waves), 25.2-27.1 ms for the last at 1 M and 2 M (it
-// then runs one sample at a time). At 2^23 slots the path state is 2.1 GB, of 180.
+// then runs one sample at a time). At 2^23 slots the path state is 2.35 GB (2.68 with the adjoint's), of 180.
 struct WavePlan
 {
     std::vector<uint32_t> table;     // per wave: entries (view | sample of the wave << 16), then item bases

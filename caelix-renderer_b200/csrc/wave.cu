@@ -1015,8 +1015,9 @@ __global__ void __launch_bounds__(kWaveThreads, kMinBlocks)
 
 namespace {
 
-// Carves the wave buffers from `base` (null: only the size is wanted); returns the bytes.
-uint64_t carve(char* base, uint32_t capacity, WaveBuffers& b)
+// Carves the wave buffers from `base` (null: only the size is wanted); returns the bytes: 280 a slot, and 40
+// for the adjoint's arrays where they are wanted.
+uint64_t carve(char* base, uint32_t capacity, bool adjoint, WaveBuffers& b)
 {
     const uint64_t c = std::max<uint32_t>(capacity, 32);
     uint64_t at = 0;
@@ -1048,24 +1049,26 @@ uint64_t carve(char* base, uint32_t capacity, WaveBuffers& b)
     take(b.neeq, c);
     take(b.lampq, c);
     take(b.counts, kCountWords);
-    take(b.adj_g, c);
-    take(b.adj_r, c);
-    take(b.adj_nee, c);
+    if (adjoint) {
+        take(b.adj_g, c);
+        take(b.adj_r, c);
+        take(b.adj_nee, c);
+    }
     return at;
 }
 
 }  // namespace
 
-uint64_t wave_buffer_bytes(uint32_t capacity)
+uint64_t wave_buffer_bytes(uint32_t capacity, bool adjoint)
 {
     WaveBuffers b;
-    return carve(nullptr, capacity, b);
+    return carve(nullptr, capacity, adjoint, b);
 }
 
-WaveBuffers wave_carve(void* base, uint32_t capacity)
+WaveBuffers wave_carve(void* base, uint32_t capacity, bool adjoint)
 {
     WaveBuffers b;
-    carve(static_cast<char*>(base), capacity, b);
+    carve(static_cast<char*>(base), capacity, adjoint, b);
     return b;
 }
 
