@@ -889,11 +889,12 @@ __global__ void group_occupancy_kernel(const int32_t* __restrict__ keys, uint32_
                                        uint32_t* __restrict__ flags)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t with_brick = __ballot_sync(0xFFFFFFFFu, i < n);  // the lanes that reach the match
     if (i >= n) return;
     // One lane per run of bricks of one group (neighbours in linear order mostly share it): a thread per
     // brick asking the flag's word took 31 us over 100 k bricks of 72 groups.
     const uint32_t g = brick_group(keys, i, gg.origin, gg.groups, gg.shift);
-    const uint32_t peers = __match_any_sync(__activemask(), g);
+    const uint32_t peers = __match_any_sync(with_brick, g);
     if ((threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1u && !(flags[g] & kGroupOccupied))
         atomicOr(&flags[g], kGroupOccupied);
 }
