@@ -353,21 +353,29 @@ __global__ void __launch_bounds__(kWaveThreads)
     counter.finish(views);
 }
 
-// The rays after the camera's of a large wave (world bricks only). They differ widely in length: with a ray per lane from
-// start to end 4 of 32 lanes were active on average on a 300 k-brick world. Here a lane that has
-// finished waits until kRefill lanes have; these write their results and take the next rays of the
-// queue together. A lane walks at most kWalkCells empty cells before the lanes that have reached a
-// brick test theirs. Measured against a ray per lane (one B200): 1920 x 1080 x 4 spp on 300 k bricks
-// 14.1 -> 12.1 ms (7.3 lanes), 333 x 251 x 8 spp 0.88 -> 0.78, 12 views of 256 and 512 squared 5.86 ->
-// 5.26, 512 x 512 0.458 -> 0.453; 160 x 90 0.124 -> 0.133 (nothing to refill from: small waves keep a ray
-// per lane). kRefill of 6 and 20: 12.3 and 12.4 ms on the first; kWalkCells of 3, 8, 64: 12.4, 12.2, 12.8 there
-// and 2.06, 1.97, 1.94 on the adjoint of a world without empty bricks. A pool of 64 rays per warp in
-// shared memory, taken up in phases of one kind (10 lanes, but the rays' state through shared memory
-// in every phase): 11.8, 0.84, 5.13 and 0.547 ms. Eight CTAs per SM instead of six: 12.3 ms. Camera rays, whose
-// neighbours walk alike, are faster with a ray per lane (1.18 against 1.56 ms for 8.3 M).
+// The rays after the camera's of a large wave (world bricks only: there is no entity traversal here). They differ widely
+// in length: with a ray per lane from start to end 4 of 32 lanes are active on average on a 300 k-brick world. Here a
+// lane that has finished waits until kRefill lanes have; these write their results and take the next rays of the
+// queue together (7.3 lanes). A lane walks at most kWalkCells empty cells before the lanes that have reached a
+// brick test theirs. kRefill of 6 and 20 instead of 12: 1920 x 1080 x 4 spp on 300 k bricks 12.3 and 12.4 against 12.1
+// ms; kWalkCells of 3, 8, 64: 12.4, 12.2, 12.8. A pool of 64 rays per warp in shared memory, taken up in phases of
+// one kind (10 lanes, but the rays' state through shared memory in every phase): 11.8, but 0.547 against 0.453 for
+// 512 x 512. Eight CTAs per SM instead of six: 12.3. Camera rays, whose neighbours walk alike, are faster with a ray
+// per lane (1.18 against 1.56 ms for 8.3 M).
+//
+// Refilling needs a long queue: in the later bounces of a small wave there is nothing to refill from. Frame times with a
+// ray per lane over those with refilling (one B200; cubes of 300, 5,000 and 40,000 bricks, terrains of 20,000 and
+// 150,000), by paths of the wave:
+//   2 bounces:  130 k 0.90 0.97 0.99 0.94 1.01   345 k 0.94 0.99 1.01 1.01 1.04
+//   3 bounces:  600 k 0.96 1.02 1.03 0.99 1.06   1 M   0.98 1.03 1.06 1.04 1.09   8 M 1.02 1.09 1.11 1.11 1.16
+//   5 bounces:  130 k 0.84 0.89 0.94 0.86 0.91   345 k 0.89 0.94 0.97 0.93 0.98
+//   6 bounces:  600 k 0.91 0.97 0.99 0.94 1.00   1 M   0.94 1.02 1.04 1.00 1.06   8 M 1.01 1.09 1.10 1.09 1.15
+// The geometric mean over 1, 3 and 6 bounces is 0.985 at 420 k, 0.99 at 600 k and 1.02 at 1 M. Neighbours in a wave of
+// several views walk less alike (4 to 8 views, 3 bounces): 164 k 0.96, 200 k 1.02, 369 k 1.03, 400 k 1.05.
 constexpr uint32_t kRefill = 12;
 constexpr uint32_t kWalkCells = 8;
-constexpr uint32_t kRefillPaths = 1u << 17;  // waves of more paths than this are traced so
+// Waves of more paths than this are traced so, of one view and of several.
+constexpr uint32_t kRefillPaths = 640'000, kRefillPathsViews = 180'000;
 
 __global__ void __launch_bounds__(kWaveThreads, 6)
     wave_trace_refill_kernel(const WaveView* __restrict__ views, const WaveBuffers b, uint32_t parity, bool one_view)
@@ -1197,7 +1205,7 @@ cudaError_t wave_run(const WaveView* d_views, const WavePlan& plan, const uint32
                                                            sm_count * (uint32_t)light_blocks[entities ? 1 : 0]);
             const bool one_view = plan.one_view;
             const bool quad = n <= kQuadPaths;
-            const bool refill = !entities && n > kRefillPaths;
+            const bool refill = !entities && n > (one_view ? kRefillPaths : kRefillPathsViews);
             const uint32_t refill_grid = sm_count * (uint32_t)refill_blocks;
             const uint32_t quad_grid = std::min<uint32_t>((8 * n + kWaveThreads - 1) / kWaveThreads, sm_count * 5);
             const auto stage = [&](auto with_entities, uint32_t it) {
