@@ -580,10 +580,12 @@ CAELIX_API CaelixResult caelix_renderer_render(CaelixRenderer* renderer, const C
    shader): the kernel organisation of caelix_renderer_render. Both give the same radiance, bit
    for bit.
      CAELIX_TRACE_WAVEFRONT (default): path state in device memory, one kernel per stage (trace,
-       shade) over compacted ray and path queues, every bounce; wave_capacity bounds the paths in
-       flight (0 = one per pixel, or one per pixel and sample while that is at most 2^23 and its path
+       shade, light) over compacted queues, every bounce; wave_capacity bounds the paths in flight
+       (0 = one per pixel, or one per pixel and sample while that is at most 2^23 and its path
        state fits the device; else at least 32), the rest of the pixels and samples follow in later
-       waves. A size that did not fit is not asked for again until the mode is set again.
+       waves. A path's state takes 280 bytes (320 in caelix_renderer_backward), up to 2.35 GB that
+       the renderer keeps; a smaller wave_capacity bounds it at some cost in time. A size that did
+       not fit is not asked for again until the mode is set again.
      CAELIX_TRACE_MEGAKERNEL: one thread per pixel runs its whole path in one kernel. */
 #define CAELIX_TRACE_WAVEFRONT 0u
 #define CAELIX_TRACE_MEGAKERNEL 1u
@@ -722,6 +724,9 @@ CAELIX_API void caelix_batch_destroy(CaelixBatch* batch);
    host waits in between). */
 CAELIX_API CaelixResult caelix_batch_run(CaelixBatch* batch, const CaelixFrameDesc* frame);
 
+/* get_tuning gives the tuning that was set or autotuned, and for a batch with neither the persistent
+   kernel's defaults, which is not what such a batch runs (CaelixBatchTuning::kernel): setting them
+   back switches it to the persistent kernel. */
 CAELIX_API CaelixResult caelix_batch_set_tuning(CaelixBatch* batch, const CaelixBatchTuning* tuning);
 CAELIX_API CaelixResult caelix_batch_get_tuning(const CaelixBatch* batch, CaelixBatchTuning* out);
 
@@ -746,12 +751,13 @@ typedef struct CaelixBatchStats
     float gpu_ms;             /* the whole graph launch */
     uint32_t kernel_launches; /* kernel nodes of the graph */
     uint32_t light_tree_builds;
-    uint32_t wavefront;       /* persistent threads of the trace */
+    uint32_t wavefront;       /* paths in flight: the wavefront kernels' slots, or the persistent
+                                 kernel's threads */
     uint32_t graph_captures;  /* captures so far */
     uint32_t pad;
 } CaelixBatchStats;
 CAELIX_API CaelixResult caelix_batch_get_stats(CaelixBatch* batch, CaelixBatchStats* out);
-/* Rays of one view in the newest run (kernel_launches = 1: the shared persistent launch). */
+/* Rays of one view in the newest run (kernel_launches = 1: the graph launch that the views share). */
 CAELIX_API CaelixResult caelix_batch_get_view_stats(CaelixBatch* batch, uint32_t view, CaelixRenderStats* out);
 
 /* ---------------------------------------------------------------------------
