@@ -1,4 +1,6 @@
 """The device memory of a render's path state: 280 bytes a slot, without the adjoint's arrays (40 more)."""
+import gc
+
 import pytest
 
 from caelix_b200 import workloads
@@ -21,6 +23,7 @@ def test_render_keeps_no_adjoint_arrays(cuda_device):
     first.backward(d, 32, 32, vs.camera, *grads, bounces=1, seed=1, spp=2)
 
     def taken(call):
+        gc.collect()
         torch.cuda.synchronize()
         before = torch.cuda.mem_get_info()[0]
         call()
